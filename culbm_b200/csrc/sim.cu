@@ -64,7 +64,7 @@ StepArgs<S, typename ArithOf<S>::type> make_args(const culbm_sim* s, int src, in
     using R = typename ArithOf<S>::type;
     StepArgs<S, R> a{};
     long long stride = s->n;
-    if (is_blocked(s->cfg)) tiles_view(s, &a.ring_nz, &a.ring_off, &stride);
+    if (s->tiles) tiles_view(s, &a.ring_nz, &a.ring_off, &stride);
     a.dom = s->dom;
     a.ops = s->d_ops;
     a.rho = s->d_mac[0];
@@ -85,9 +85,8 @@ StepArgs<S, typename ArithOf<S>::type> make_args(const culbm_sim* s, int src, in
 // Layout of the newest state and the buffer holding it.
 int current_layout(const culbm_sim* s)
 {
-    if (s->cfg.stream_policy == CULBM_STREAM_INPLACE && !is_blocked(s->cfg))
-        return s->aa_phase == 0 ? LAYOUT_AA_A : LAYOUT_AA_B;
-    if (is_blocked(s->cfg) && s->cfg.use_ring_ddf_buf) return LAYOUT_PULL_RING;
+    if (s->inplace) return s->aa_phase == 0 ? LAYOUT_AA_A : LAYOUT_AA_B;
+    if (s->cfg.use_ring_ddf_buf) return LAYOUT_PULL_RING;
     return LAYOUT_PULL;
 }
 
@@ -210,11 +209,11 @@ template <typename S>
 culbm_status fill_rest(culbm_sim* s)
 {
     using R = typename ArithOf<S>::type;
-    if (is_blocked(s->cfg)) return tiles_reset(s);
+    if (s->tiles) return tiles_reset(s);
     const dim3 g = cell_grid(s->dom), b = cell_block();
     for (int k = 0; k < s->npop; ++k) {
         auto a = make_args<S>(s, k, k);
-        if (s->cfg.stream_policy == CULBM_STREAM_INPLACE && !is_blocked(s->cfg))
+        if (s->inplace)
             k_fill_equilibrium<LAYOUT_AA_A, S, R><<<g, b, 0, s->stream>>>(a, R(1), R(0), R(0), R(0));
         else
             k_fill_equilibrium<LAYOUT_PULL, S, R><<<g, b, 0, s->stream>>>(a, R(1), R(0), R(0), R(0));
@@ -247,7 +246,7 @@ bool rows_applicable(const culbm_sim* s)
     if (is_blocked(s->cfg) || s->esize != 2) return false;
     if (s->cfg.kernel_variant != 1 && s->cfg.kernel_variant != 2) return false;
     if (D.nx % 16 != 0 || D.nx < 32 || D.nx > 992) return false;
-    if (s->cfg.stream_policy == CULBM_STREAM_INPLACE && (D.ny < 3 || D.nz < 3)) return false;
+    if (s->inplace && (D.ny < 3 || D.nz < 3)) return false;
     return true;
 }
 
@@ -283,7 +282,7 @@ culbm_status rows_setup(culbm_sim* s)
     if constexpr (Is16<S>::value) {
         CULBM_TRY(with_row_shape(s, [&](auto ns, auto ob, auto pf) -> culbm_status {
             constexpr int NS = decltype(ns)::value, OB = decltype(ob)::value, PF = decltype(pf)::value;
-            if (s->cfg.stream_policy == CULBM_STREAM_PULL) {
+            if (!s->inplace) {
                 CULBM_TRY((rows_prepare<S, ROWS_PULL, NS, OB, PF>(s)));
             } else {
                 CULBM_TRY((rows_prepare<S, ROWS_AA_ODD, NS, OB, PF>(s)));
@@ -424,7 +423,7 @@ culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
             }
             if (s->rows) {
                 const Domain& D = s->dom;
-                if (s->cfg.stream_policy == CULBM_STREAM_PULL) {
+                if (!s->inplace) {
                     auto a = make_args<S>(s, s->cur, 1 - s->cur);
                     a.seed = seed;
                     CULBM_TRY((rows_launch<S, ROWS_PULL>(s, a, 0, 0, D.ny, D.nz)));
@@ -452,7 +451,7 @@ culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
                 continue;
             }
         }
-        if (s->cfg.stream_policy == CULBM_STREAM_PULL) {
+        if (!s->inplace) {
             auto a = make_args<S>(s, s->cur, 1 - s->cur);
             a.seed = seed;
             k_pull_step<S, R><<<g, b, 0, s->stream>>>(a, 0);
@@ -580,15 +579,6 @@ culbm_status upload_state(culbm_sim* s, const uint32_t* flag, const float* const
     }
     k_build_ops<<<cell_grid(s->dom), cell_block(), 0, s->stream>>>(s->dom, s->d_flag, s->d_ops, 0);
     CULBM_CUDA(cudaGetLastError());
-    if (is_blocked(s->cfg)) {
-        std::vector<uint32_t> host;
-        const uint32_t* hf = flag;
-        if (hf == nullptr) {
-            host.assign(static_cast<size_t>(n), kDefaultFlag);
-            hf = host.data();
-        }
-        CULBM_TRY(tiles_upload_flags(s, hf));
-    }
     CULBM_TRY(with_storage(s, [&](auto tag) { return fill_rest<typename decltype(tag)::type>(s); }));
     s->step = 0;
     s->loaded = true;
@@ -693,7 +683,7 @@ culbm_status run_slab_steps(culbm_sim* s, int nslab, int nstream, int t0, int t1
     auto ev = [&](int j, int k) { return s->slab_ev[static_cast<size_t>(j) * kSlabEvents + k]; };
     auto planes = [&](int za, int zb) { return dim3((D.nx + 31) / 32, (D.ny + 7) / 8, zb - za); };
     const dim3 b = cell_block();
-    const bool pull = s->cfg.stream_policy == CULBM_STREAM_PULL;
+    const bool pull = !s->inplace;
 
     struct Task {
         int d, t, j;   // t = t0 - 1: op bytes; t1: dump
@@ -822,7 +812,7 @@ culbm_status run_host_overlapped(culbm_sim* s, const uint32_t* flag, const float
     // Slab by slab for the first and the last nslab steps, which the copies
     // overlap; whole-domain launches in between.  fill_rest left cur = 0 and
     // aa_phase = 0.
-    const bool pull = s->cfg.stream_policy == CULBM_STREAM_PULL;
+    const bool pull = !s->inplace;
     int shift_end = T;   // steps into the skewed phase that ends with the dumps
     if (T <= 2 * nslab) {
         CULBM_TRY(run_slab_steps<S>(s, nslab, nstream, 0, T, true, true));
@@ -926,9 +916,9 @@ culbm_status culbm_create(const culbm_config* cfg, culbm_sim** out)
         CULBM_CUDA(cudaEventCreate(&s->ev0));
         CULBM_CUDA(cudaEventCreate(&s->ev1));
         const long long n = s->n;
-        const bool blocked = is_blocked(s->cfg);
-        const bool inplace = s->cfg.stream_policy == CULBM_STREAM_INPLACE && !blocked;
-        s->npop = (inplace || (blocked && s->cfg.use_ring_ddf_buf)) ? 1 : 2;
+        const bool inplace = s->cfg.stream_policy == CULBM_STREAM_INPLACE && !is_blocked(s->cfg);
+        s->inplace = inplace;
+        s->npop = (inplace || s->cfg.use_ring_ddf_buf) ? 1 : 2;
 
         // Capacity check before allocating: populations dominate.
         size_t free_b = 0, total_b = 0;
@@ -942,7 +932,7 @@ culbm_status culbm_create(const culbm_config* cfg, culbm_sim** out)
         CULBM_TRY(dev_alloc(s, reinterpret_cast<void**>(&s->d_ops), n, "op bytes"));
         for (int k = 0; k < 4; ++k)
             CULBM_TRY(dev_alloc(s, reinterpret_cast<void**>(&s->d_mac[k]), n * sizeof(float), "macroscopic buffer"));
-        if (!blocked || !s->cfg.use_ring_ddf_buf) {
+        if (!s->cfg.use_ring_ddf_buf) {
             for (int k = 0; k < s->npop; ++k)
                 CULBM_TRY(dev_alloc(s, &s->d_pop[k], 27ull * n * s->esize, "populations"));
         }
@@ -961,7 +951,7 @@ culbm_status culbm_create(const culbm_config* cfg, culbm_sim** out)
         s->red_blocks = 592;
         CULBM_TRY(dev_alloc(s, reinterpret_cast<void**>(&s->d_red), (4ull * s->red_blocks + 4) * sizeof(double),
                             "reduction scratch"));
-        if (blocked) CULBM_TRY(tiles_create(s));
+        if (uses_tile_engine(s->cfg)) CULBM_TRY(tiles_create(s));
         CULBM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->err_host), sizeof(int), cudaHostAllocMapped));
         *s->err_host = 0;
         CULBM_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->err_dev), s->err_host, 0));
@@ -1042,7 +1032,7 @@ culbm_status culbm_step(culbm_sim* sim, uint32_t nsteps)
 {
     CULBM_TRY(check_sim(sim, true));
     if (nsteps == 0) return CULBM_OK;
-    if (is_blocked(sim->cfg)) {
+    if (sim->tiles) {
         CULBM_TRY(tiles_step(sim, nsteps));
     } else {
         CULBM_TRY(with_storage(sim, [&](auto tag) { return plain_steps<typename decltype(tag)::type>(sim, nsteps); }));
@@ -1110,7 +1100,7 @@ culbm_status culbm_run_host(culbm_sim* sim, const uint32_t* flag, const float* r
     for (float* o : out)
         if (o == nullptr) return fail(CULBM_ERR_INVALID_ARGUMENT, "culbm_run_host: NULL output buffer");
     const float* mac[4] = {rho, vx, vy, vz};
-    if (is_blocked(sim->cfg) || sim->rows || sim->warp_pull) {
+    if (sim->tiles || sim->rows || sim->warp_pull) {
         // The tile engine and the staged 16-bit kernels step the whole domain at once.
         CULBM_TRY(upload_state(sim, flag, mac));
         CULBM_TRY(culbm_step(sim, nsteps));

@@ -62,6 +62,7 @@ struct culbm_sim {
     culbm::EdgeLayout el{};
     long long edge_elems = 0;
     size_t esize = 4;               // bytes per stored population
+    bool inplace = false;           // AA pattern in one buffer; else a double buffer (or the ring)
     double* d_red = nullptr;        // reduction partials
     int red_blocks = 0;
 
@@ -134,7 +135,6 @@ culbm_status dev_alloc(culbm_sim* s, void** p, size_t bytes, const char* what);
 culbm_status validate_blocking(const culbm_config& cfg);
 culbm_status tiles_create(culbm_sim* sim);
 void tiles_destroy(culbm_sim* sim);
-culbm_status tiles_upload_flags(culbm_sim* sim, const uint32_t* host_flag);
 culbm_status tiles_reset(culbm_sim* sim);
 culbm_status tiles_step(culbm_sim* sim, uint32_t nsteps);
 // Where the newest global state lives: ring planes (0 = plain buffers), its
@@ -142,5 +142,7 @@ culbm_status tiles_step(culbm_sim* sim, uint32_t nsteps);
 void tiles_view(const culbm_sim* sim, int* ring_nz, int* offz, long long* stride);
 void tiles_info(const culbm_sim* sim, culbm_info* info);
 bool is_blocked(const culbm_config& cfg);
+// Whether a blocked policy runs on the tile or cluster engine.
+bool uses_tile_engine(const culbm_config& cfg);
 
 }  // namespace culbm

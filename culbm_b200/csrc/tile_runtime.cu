@@ -6,12 +6,14 @@
 // Replaces the reference's haloBlocking*Run lambdas and initBlockingFlag /
 // initRingDDFBuf / mapGlobalMem2PersistL2
 // (src/simulator/single_dev_expt/simulator_expt_platform.cu:120-305, 608-942).
-// optPolicy 1 (static L2) runs on the same L2 tile engine as 3 (dynamic L2).
+// optPolicy 1 (static L2) and 3 (dynamic L2) run on the L2 tile engine when
+// they use the ring buffer or the persisting-L2 window and as plain pull
+// steps otherwise (uses_tile_engine).
 // optPolicy 2 (L1/L2 mixed) with pull streaming runs on the cluster engine
 // (cluster_kernels.cuh: one thread-block cluster per tile, populations in
 // registers, streaming through shared memory and DSMEM, one launch per
-// round) whenever the tile fits one cluster; larger tiles, and in-place
-// streaming, run on the L2 tile engine.  Every engine gives the plain step's
+// round) whenever the tile fits one cluster; larger tiles run on the L2 tile
+// engine.  Every engine gives the plain step's
 // results bit for bit, so they differ only in speed.
 #include <algorithm>
 #include <climits>
@@ -103,6 +105,22 @@ struct TileState {
 };
 
 bool is_blocked(const culbm_config& cfg) { return cfg.opt_policy != CULBM_OPT_NONE; }
+
+// Which blocked configurations run on the engines of this file.  Every policy
+// gives the plain step's bits, and the double-buffered ones keep the state as
+// the plain pull does, so the choice is one of speed.  B200's L2 copies only
+// twice as fast as its HBM: at 288x272x280 the tile engine reached 15.0k
+// MLUPS with the README tile (FP32) and at most 24.3k with any, the plain
+// pull 29.7k; FP16-SR tiles 19.2k against 38.7k.  The tile engine stays where
+// the caller asks for something only it does: the ring buffer (one population
+// buffer), the persisting-L2 window, and optPolicy 2 with pull streaming (its
+// cluster engine, or L2 tiles where no cluster holds the tile).
+bool uses_tile_engine(const culbm_config& cfg)
+{
+    if (!is_blocked(cfg)) return false;
+    return cfg.use_ring_ddf_buf || cfg.persist_l2 ||
+           (cfg.opt_policy == CULBM_OPT_L1L2 && cfg.stream_policy == CULBM_STREAM_PULL);
+}
 
 namespace {
 
@@ -639,8 +657,6 @@ void tiles_destroy(culbm_sim* s)
     s->tiles = nullptr;
 }
 
-culbm_status tiles_upload_flags(culbm_sim*, const uint32_t*) { return CULBM_OK; }
-
 // Resets the round state and fills the global state with rest equilibrium.
 culbm_status tiles_reset(culbm_sim* s)
 {
@@ -676,13 +692,13 @@ void tiles_view(const culbm_sim* s, int* ring_nz, int* offz, long long* stride)
 
 void tiles_info(const culbm_sim* s, culbm_info* info)
 {
-    const TileState* ts = s->tiles;
-    if (ts == nullptr) return;
+    const culbm_config& c = s->cfg;
+    if (!is_blocked(c)) return;
     for (int k = 0; k < 3; ++k) {
-        info->blocking_num[k] = static_cast<uint32_t>(ts->nt[k]);
-        info->blocking_dim[k] = static_cast<uint32_t>(ts->B[k]);
+        info->blocking_dim[k] = c.block_dim[k] * c.grid_dim[k];
+        info->blocking_num[k] = blk_num(c.domain_dim[k], info->blocking_dim[k], static_cast<uint32_t>(c.inner_loop));
     }
-    info->persisting_l2_bytes = ts->persist_bytes;
+    info->persisting_l2_bytes = s->tiles ? s->tiles->persist_bytes : 0;
 }
 
 }  // namespace culbm

@@ -116,6 +116,34 @@ def test_blocked_fp64_and_moments(culbm, orc):
                 assert np.array_equal(bits(sim.field(k)), bits(w)), (ring, k)
 
 
+@pytest.mark.parametrize("storage", ["fp32", "fp16sr", "fp64"])
+@pytest.mark.parametrize("sp,op", [(0, 1), (0, 3), (1, 1), (1, 2), (1, 3)])
+def test_blocked_engine_choice(culbm, storage, sp, op):
+    """Double-buffered blocked policies run as plain pull steps, one launch
+    each, with the plain pull's bits (inactive cells, steps in several calls,
+    run_host); with the persisting-L2 window they run on the tile engine."""
+    sc = S.reference_channel_cube(37, 26, 22, 0.05)
+    rng = np.random.default_rng(op)
+    sc.flag[rng.random(sc.flag.shape) < 0.03] = 0
+    dtype = np.float64 if storage == "fp64" else np.float32
+    with culbm.Simulation(sc.shape, inv_tau=0.6, storage=storage) as sim:
+        want_fields = sim.run_host(8, *sc.arrays())
+        want = sim.pulled_ddf(dtype)
+    for persist in (False, True):
+        with culbm.Simulation(sc.shape, stream_policy=sp, opt_policy=op, inv_tau=0.6, inner_loop=3, tile=(16, 14, 12),
+                              storage=storage, persist_l2=persist) as sim:
+            sim.load_state(*sc.arrays())
+            sim.step(3)
+            sim.step(5)
+            launches = sim.info()["launches_per_step"]
+            assert launches > 2.0 if persist else launches == 1.0
+            if persist:   # tiles keep leftovers in cells without STORE
+                continue
+            assert np.array_equal(bits(sim.pulled_ddf(dtype)), bits(want))
+            for a, b in zip(sim.run_host(8, *sc.arrays()), want_fields):
+                assert np.array_equal(bits(a), bits(b))
+
+
 def _valid_axis(dom, blk, it):
     """blocking_core::validBlkAxisConfig and the engine's extra check (the
     tile must be large enough for innerLoop when more than two are needed)."""
