@@ -15,6 +15,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cells2_kernels.cuh"
 #include "row_kernels.cuh"
 #include "warp_kernels.cuh"
 #include "sim_internal.cuh"
@@ -389,11 +390,68 @@ culbm_status warp_pull_setup(culbm_sim* s)
     return CULBM_OK;
 }
 
+// Whether the 16-bit format S steps two cells per thread (cells2_kernels.cuh).
+template <typename S>
+bool two_cells(const Domain& D)
+{
+    return Is16<S>::value && D.nx % 2 == 0;
+}
+
+// One pull step of the planes [za, zb) in the arguments' buffers.
+template <typename S, typename R>
+culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t st)
+{
+    const Domain& D = a.dom;
+    bool done = false;
+    if constexpr (Is16<S>::value) {
+        if (two_cells<S>(D)) {
+            FastDiv row;
+            row.set(static_cast<uint32_t>(D.nx));
+            const long long per_block = 2ll * kCells2Threads;
+            const dim3 g(static_cast<unsigned>((D.nxy + per_block - 1) / per_block), zb - za);
+            k_pull_cells2<S><<<g, kCells2Threads, 0, st>>>(a, row, za, kNegZero2);
+            done = true;
+        }
+    }
+    if (!done)
+        k_pull_step<S, R><<<dim3((D.nx + 31) / 32, (D.ny + 7) / 8, zb - za), cell_block(), 0, st>>>(a, za);
+    CULBM_CUDA(cudaGetLastError());
+    return CULBM_OK;
+}
+
+// One in-place step of the planes [za, zb) (odd: layout A -> B).
+template <typename S, typename R>
+culbm_status launch_inplace(const StepArgs<S, R>& a, bool odd, int za, int zb, cudaStream_t st)
+{
+    const Domain& D = a.dom;
+    bool done = false;
+    if constexpr (Is16<S>::value) {
+        if (two_cells<S>(D)) {
+            long long blocks = 0;
+            const Cells2Grid g = cells2_grid(D, za, zb, &blocks);
+            if (odd) k_aa_odd_cells2<S><<<static_cast<unsigned>(blocks), kCells2Threads, 0, st>>>(a, g, kNegZero2);
+            else k_aa_even_cells2<S><<<static_cast<unsigned>(blocks), kCells2Threads, 0, st>>>(a, g, kNegZero2);
+            done = true;
+        }
+    }
+    if (!done && za == 0 && zb == D.nz) {
+        const dim3 g = split_grid(D, AaShape<S>::rows, AaShape<S>::cols);
+        if (odd) k_aa_odd<S, R><<<g, aa_block<S>(), 0, st>>>(a);
+        else k_aa_even<S, R><<<g, aa_block<S>(), 0, st>>>(a);
+    } else if (!done) {
+        const SlabSplit q = slab_split(D, za, zb, AaShape<S>::rows);
+        const dim3 g = slab_split_grid(D, q, AaShape<S>::rows, AaShape<S>::cols);
+        if (odd) k_aa_odd_slab<S, R><<<g, aa_block<S>(), 0, st>>>(a, q);
+        else k_aa_even_slab<S, R><<<g, aa_block<S>(), 0, st>>>(a, q);
+    }
+    CULBM_CUDA(cudaGetLastError());
+    return CULBM_OK;
+}
+
 template <typename S>
 culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
 {
     using R = typename ArithOf<S>::type;
-    const dim3 g = cell_grid(s->dom), b = cell_block();
     for (uint32_t k = 0; k < nsteps; ++k) {
         const uint32_t seed = step_seed(static_cast<uint32_t>(s->step + k));
         if constexpr (Is16<S>::value) {
@@ -454,18 +512,12 @@ culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
         if (!s->inplace) {
             auto a = make_args<S>(s, s->cur, 1 - s->cur);
             a.seed = seed;
-            k_pull_step<S, R><<<g, b, 0, s->stream>>>(a, 0);
-            CULBM_CUDA(cudaGetLastError());
+            CULBM_TRY((launch_pull<S, R>(a, 0, s->dom.nz, s->stream)));
             s->cur ^= 1;
         } else {
             auto a = make_args<S>(s, 0, 0);
             a.seed = seed;
-            const dim3 gs = split_grid(s->dom, AaShape<S>::rows, AaShape<S>::cols);
-            if (s->aa_phase == 0)
-                k_aa_odd<S, R><<<gs, aa_block<S>(), 0, s->stream>>>(a);
-            else
-                k_aa_even<S, R><<<gs, aa_block<S>(), 0, s->stream>>>(a);
-            CULBM_CUDA(cudaGetLastError());
+            CULBM_TRY((launch_inplace<S, R>(a, s->aa_phase == 0, 0, s->dom.nz, s->stream)));
             s->aa_phase ^= 1;
         }
         s->launches += 1;
@@ -728,18 +780,12 @@ culbm_status run_slab_steps(culbm_sim* s, int nslab, int nstream, int t0, int t1
             if (pull) {
                 auto a = make_args<S>(s, t & 1, 1 - (t & 1));
                 a.seed = step_seed(static_cast<uint32_t>(t));
-                k_pull_step<S, R><<<planes(za, zb), b, 0, st>>>(a, za);
+                CULBM_TRY((launch_pull<S, R>(a, za, zb, st)));
             } else {
                 auto a = make_args<S>(s, 0, 0);
                 a.seed = step_seed(static_cast<uint32_t>(t));
-                constexpr int ar = AaShape<S>::rows, ac = AaShape<S>::cols;
-                const SlabSplit q = slab_split(D, za, zb, ar);
-                if ((t & 1) == 0)
-                    k_aa_odd_slab<S, R><<<slab_split_grid(D, q, ar, ac), aa_block<S>(), 0, st>>>(a, q);
-                else
-                    k_aa_even_slab<S, R><<<slab_split_grid(D, q, ar, ac), aa_block<S>(), 0, st>>>(a, q);
+                CULBM_TRY((launch_inplace<S, R>(a, (t & 1) == 0, za, zb, st)));
             }
-            CULBM_CUDA(cudaGetLastError());
             s->launches += 1;
         }
         CULBM_CUDA(cudaEventRecord(ev(j, t & 3), st));

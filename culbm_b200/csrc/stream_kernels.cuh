@@ -244,15 +244,11 @@ __device__ __forceinline__ CellCoord cell_of_thread(const Domain& D, int z0 = 0)
     return c;
 }
 
-// One pull step src -> dst over the planes z0 .. z0 + gridDim.z - 1 (the
-// whole domain with z0 = 0 and a cell_grid launch).
+// The pull step of one cell, src -> dst.
 // Replaces StaticD3Q27PullKernel, reference kernel.cu:2489-2632.
 template <typename S, typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
-    k_pull_step(const __grid_constant__ StepArgs<S, R> a, int z0)
+__device__ __forceinline__ void pull_cell(const StepArgs<S, R>& a, const CellCoord c)
 {
-    const CellCoord c = cell_of_thread(a.dom, z0);
-    if (!c.valid) return;
     const uint8_t op = a.ops[c.i];
     R f[27];
     if (op & OP_LOAD) {
@@ -264,6 +260,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
     cell_update_for<S, true>(op, a.inv_tau, a.rho, a.vx, a.vy, a.vz, c.i, f);
     if (op & OP_STORE)
         put27_raw<S>(f, cell_hash(static_cast<uint32_t>(c.i), a.seed), [&](int d) { return a.dst.p[d] + c.i; });
+}
+
+// One pull step over the planes z0 .. z0 + gridDim.z - 1 (the whole domain
+// with z0 = 0 and a cell_grid launch).
+template <typename S, typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
+    k_pull_step(const __grid_constant__ StepArgs<S, R> a, int z0)
+{
+    const CellCoord c = cell_of_thread(a.dom, z0);
+    if (c.valid) pull_cell<S, R>(a, c);
 }
 
 // In-place odd step (layout A -> B): each cell pulls f_d from the reversed
@@ -290,7 +296,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
 // beside the inner rows rather than as a tail; each further slice is one
 // interior z-plane of inner rows.  Rows are contiguous in x, so warp
 // accesses stay coalesced, and no thread divides by a runtime value.
-enum RowSet : int { ROWS_INNER = 0, ROWS_OUTER = 1 };
+// ROWS_INNER_ONE: a cell of an inner row on its own (no warp-wide choice).
+enum RowSet : int { ROWS_INNER = 0, ROWS_OUTER = 1, ROWS_INNER_ONE = 2 };
 
 // Block shape of the in-place step launches (split_grid, slab_split), by
 // storage format: one row of 96 cells (three warps, one 32-cell segment
@@ -368,6 +375,84 @@ __device__ __forceinline__ const S* xface_edge_ptr(const S* edge, const Domain& 
     return edge + L.off[side] + (long long)j * D.ny * D.nz + y + (long long)D.ny * z;
 }
 
+// Face rows (ROWS_OUTER) of the 16-bit formats.  Few cells take this code, and
+// it shares the instruction cache with the inner rows' code, so it selects one
+// address per pull without branches and visits the readers face by face: the
+// 32x16x16 in-place FP16-SR step takes 13.6 us against 18.5 us with the
+// per-direction branches, the 288x272x280 one the same.  FP32 and FP64 keep
+// the branches: their steps of small domains are 9 % slower this way.
+
+// Pull of layout A with the values that leave the domain from the edge buffer.
+template <typename S, typename R>
+__device__ __forceinline__ void load_face_cell(const StepArgs<S, R>& a, const CellCoord& c, R* f)
+{
+    const Domain& D = a.dom;
+    const bool xl = c.x == 0, xh = c.x == D.nx - 1, yl = c.y == 0, yh = c.y == D.ny - 1, zl = c.z == 0,
+               zh = c.z == D.nz - 1;
+    const long long nyz = 1ll * D.ny * D.nz, nxz = 1ll * D.nx * D.nz, nxy = 1ll * D.nx * D.ny;
+    const S* const ex = a.edge + (c.y + 1ll * D.ny * c.z);
+    const S* const ey = a.edge + (c.x + 1ll * D.nx * c.z);
+    const S* const ez = a.edge + (c.x + 1ll * D.nx * c.y);
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
+        const bool ox = cx == 1 ? xl : cx == -1 ? xh : false, oy = cy == 1 ? yl : cy == -1 ? yh : false,
+                   oz = cz == 1 ? zl : cz == -1 ? zh : false;
+        const S* p = a.src.p[26 - d] + (c.i - nb_off(D, d));
+        if (oz) p = ez + (a.el.off[cz == 1 ? 4 : 5] + ((cx + 1) + 3 * (cy + 1)) * nxy);
+        if (oy) p = ey + (a.el.off[cy == 1 ? 2 : 3] + ((cx + 1) + 3 * (cz + 1)) * nxz);
+        if (ox) p = ex + (a.el.off[cx == 1 ? 0 : 1] + ((cy + 1) + 3 * (cz + 1)) * nyz);
+        f[d] = ld_stream_raw<S, R>(p);
+    }
+}
+
+// Visits the clamp readers of cell c: fn(d, f_d, y) for each direction d and
+// boundary cell y whose clamped pull of d reads c (for_each_clamp_reader).
+// A cell on one face has readers on that face only, for the nine directions
+// that leave through it; the subsets of two or three axes, for cells on an
+// edge of the domain, go through a rolled loop.
+template <typename R, class F>
+__device__ __forceinline__ void visit_clamp_readers(const Domain& D, const CellCoord& c, const R* f, F&& fn)
+{
+    const bool xl = c.x == 0, xh = c.x == D.nx - 1, yl = c.y == 0, yh = c.y == D.ny - 1, zl = c.z == 0,
+               zh = c.z == D.nz - 1;
+    auto face = [&](bool on, int axis, int side) {   // directions with component `side` along `axis`
+        if (!on) return;
+#pragma unroll
+        for (int d = 0; d < 27; ++d) {
+            const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
+            if ((axis == 0 ? cx : axis == 1 ? cy : cz) != side) continue;
+            const int yx = axis == 0 ? c.x : c.x + cx, yy = axis == 1 ? c.y : c.y + cy, yz = axis == 2 ? c.z : c.z + cz;
+            if (inside(D, yx, yy, yz)) fn(d, f[d], yx, yy, yz);
+        }
+    };
+    face(xl, 0, 1);
+    face(xh, 0, -1);
+    face(yl, 1, 1);
+    face(yh, 1, -1);
+    face(zl, 2, 1);
+    face(zh, 2, -1);
+    if ((xl || xh ? 1 : 0) + (yl || yh ? 1 : 0) + (zl || zh ? 1 : 0) < 2) return;
+    int n = 27;
+    asm volatile("" : "+r"(n));   // keeps the loop rolled
+#pragma unroll 1
+    for (int d = 0; d < n; ++d) {
+        const int cx = d % 3 - 1, cy = d / 3 % 3 - 1, cz = d / 9 - 1;
+        const int leave = ((cx == 1 && xl) || (cx == -1 && xh) ? 1 : 0) | ((cy == 1 && yl) || (cy == -1 && yh) ? 2 : 0) |
+                          ((cz == 1 && zl) || (cz == -1 && zh) ? 4 : 0);
+        if ((leave & (leave - 1)) == 0) continue;
+        R v = f[0];
+#pragma unroll
+        for (int e = 1; e < 27; ++e) v = d == e ? f[e] : v;
+#pragma unroll 1
+        for (int m = leave; m > 2; m = (m - 1) & leave) {   // the subsets of two or three leaving axes
+            if ((m & (m - 1)) == 0) continue;
+            const int yx = (m & 1) ? c.x : c.x + cx, yy = (m & 2) ? c.y : c.y + cy, yz = (m & 4) ? c.z : c.z + cz;
+            if (inside(D, yx, yy, yz)) fn(d, v, yx, yy, yz);
+        }
+    }
+}
+
 template <typename S, typename R, int ROWS>
 __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellCoord c)
 {
@@ -377,13 +462,13 @@ __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellC
     // Warps without an x-face lane (all but the first and last of a row) take
     // the straight path; the choice is uniform across the warp.
     const int xw = c.x - (threadIdx.x & 31);
-    const bool xface = ROWS == ROWS_INNER && (xw == 0 || xw + 31 >= D.nx - 1);
+    const bool xface = ROWS == ROWS_INNER_ONE || (ROWS == ROWS_INNER && (xw == 0 || xw + 31 >= D.nx - 1));
     R f[27];
     if (op & OP_LOAD) {
         if (ROWS == ROWS_INNER && !xface) {
 #pragma unroll
             for (int d = 0; d < 27; ++d) f[d] = ld_stream_raw<S, R>(a.src.p[26 - d] + (c.i - nb_off(D, d)));
-        } else if (ROWS == ROWS_INNER) {
+        } else if (ROWS != ROWS_OUTER) {
             // A warp with an x-face lane loads like the others, the face lane
             // from its own column for the directions whose source lies
             // outside (so every load stays in the domain), and that lane
@@ -404,7 +489,10 @@ __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellC
                 for (int d = 0; d < 27; d += 3) f[d] = ld_stream_raw<S, R>(xface_edge_ptr(a.edge, D, a.el, 1, d, c.y, c.z));
             }
         } else {
-            load_pulled<LAYOUT_AA_A, true>(a, c.x, c.y, c.z, c.i, true, f);
+            if constexpr (Is16<S>::value)
+                load_face_cell(a, c, f);
+            else
+                load_pulled<LAYOUT_AA_A, true>(a, c.x, c.y, c.z, c.i, true, f);
         }
     } else {
 #pragma unroll
@@ -414,7 +502,7 @@ __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellC
     if (!(op & OP_STORE)) return;
     if (ROWS == ROWS_INNER && !xface) {
         put27_raw<S>(f, hc, [&](int d) { return a.dst.p[d] + (c.i + nb_off(D, d)); });
-    } else if (ROWS == ROWS_INNER) {
+    } else if (ROWS != ROWS_OUTER) {
         // streaming target x + c_d, unless it leaves the domain in x
         const bool lo = c.x == 0, hi = c.x == D.nx - 1;
         put27_raw_if<S>(f, hc, [&](int d) { return a.dst.p[d] + (c.i + nb_off(D, d)); },
@@ -429,14 +517,22 @@ __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellC
             for (int d = 0; d < 27; d += 3) put_raw(a.dst.p[d] + (c.i + nb_off(D, d) + 1), f[d], hc, d);
         }
     } else {
-        for_dirs([&](auto dd) {
-            constexpr int d = decltype(dd)::value;
-            if (inside(D, c.x + cx_of(d), c.y + cy_of(d), c.z + cz_of(d)))
-                put_raw(a.dst.p[d] + (c.i + nb_off(D, d)), f[d], hc, d);
-            for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
-                put_raw(a.dst.p[d] + (yx + D.nx * (yy + D.ny * yz)), f[d], hc, d);
+        if constexpr (Is16<S>::value) {
+            put27_raw_if<S>(f, hc, [&](int d) { return a.dst.p[d] + (c.i + nb_off(D, d)); },
+                            [&](int d) { return inside(D, c.x + cx_of(d), c.y + cy_of(d), c.z + cz_of(d)); });
+            visit_clamp_readers(D, c, f, [&](int d, R v, int yx, int yy, int yz) {
+                put_raw(a.dst.p[d] + (yx + D.nx * (yy + D.ny * yz)), v, hc, d);
             });
-        });
+        } else {
+            for_dirs([&](auto dd) {
+                constexpr int d = decltype(dd)::value;
+                if (inside(D, c.x + cx_of(d), c.y + cy_of(d), c.z + cz_of(d)))
+                    put_raw(a.dst.p[d] + (c.i + nb_off(D, d)), f[d], hc, d);
+                for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
+                    put_raw(a.dst.p[d] + (yx + D.nx * (yy + D.ny * yz)), f[d], hc, d);
+                });
+            });
+        }
     }
 }
 
@@ -473,12 +569,18 @@ __device__ __forceinline__ void aa_even_cell(const StepArgs<S, R>& a, const Cell
                         d);
         }
     } else {
-        for_dirs([&](auto dd) {
-            constexpr int d = decltype(dd)::value;
-            for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
-                put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), f[d], hc, d);
+        if constexpr (Is16<S>::value) {
+            visit_clamp_readers(D, c, f, [&](int d, R v, int yx, int yy, int yz) {
+                put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), v, hc, d);
             });
-        });
+        } else {
+            for_dirs([&](auto dd) {
+                constexpr int d = decltype(dd)::value;
+                for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
+                    put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), f[d], hc, d);
+                });
+            });
+        }
     }
 }
 

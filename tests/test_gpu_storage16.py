@@ -57,6 +57,35 @@ def test_storage16_pull_pairs_and_x_faces(culbm, orc, storage, dims):
     assert np.array_equal(bits(got), bits(want)), (storage, dims)
 
 
+@pytest.mark.parametrize("storage", ["fp16", "bf16", "fp16sr", "bf16sr"])
+@pytest.mark.parametrize("dims", [(2, 3, 3), (4, 4, 1), (6, 1, 4), (66, 4, 3), (130, 5, 9), (258, 3, 4)])
+def test_storage16_two_cells_in_place(culbm, orc, storage, dims):
+    """The two-cells-per-thread in-place steps (even nx): rows shorter and
+    longer than a warp's pairs, fluid x- and z-faces, domains without inner
+    rows, pairs with EQU, bounce-back and non-loading cells, odd and even
+    counts; and the same steps slab by slab (run_host)."""
+    sc = S.reference_channel(*dims, 0.05)
+    sc.flag[0, :, :] = S.FLUID
+    sc.flag[:, :, 0] = S.FLUID
+    sc.flag[:, :, -1] = S.FLUID
+    rng = np.random.default_rng(sum(dims))
+    sc.flag[rng.random(sc.flag.shape) < 0.05] = S.COLLIDE | S.STORE
+    sc.flag[rng.random(sc.flag.shape) < 0.05] = S.WALL
+    sc.flag[rng.random(sc.flag.shape) < 0.03] = S.EQUILIBRIUM
+    sc.vx[:] = 0.02
+    for nsteps in (4, 5):
+        want = oracle_pulled16(orc, sc, storage, 0.7, nsteps)
+        for slabs in (0, 2, 4):
+            with culbm.Simulation(sc.shape, stream_policy=1, inv_tau=0.7, storage=storage, run_slabs=slabs) as sim:
+                if slabs:
+                    sim.run_host(nsteps, *sc.arrays())
+                else:
+                    sim.load_state(*sc.arrays())
+                    sim.step(nsteps)
+                got = sim.pulled_ddf()
+            assert np.array_equal(bits(got), bits(want)), (storage, dims, nsteps, slabs)
+
+
 def test_stochastic_rounding_is_unbiased(culbm):
     """Mean of many stochastically rounded copies of one value tends to the
     value (nearest-even would sit on one side); checked through a state
