@@ -126,6 +126,7 @@ template <typename S, typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_soft_step(const __grid_constant__ Args<S, R> a)
 {
     const CellCoord c = cell_of_thread(a.dom);
+    step_enter();
     if (!c.valid) return;
     const uint8_t op = a.ops[c.i];
     R f[27];
@@ -610,6 +611,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
     k_adj_step(const __grid_constant__ Args<S, R> a, AdjLayout L)
 {
     double gtau_local = 0.0;
+    step_enter();
     if (static_cast<int>(blockIdx.z) < L.equ_z) {
         const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
         const int k = blk * 256 + threadIdx.x + 32 * threadIdx.y;
@@ -794,8 +796,7 @@ culbm_status forward_run(culbm_adj* a, int t_begin, int t_end, S* src, SlotOf sl
         set_pops<S, R>(g.dst, dst, a->n);
         g.seed = step_seed(static_cast<uint32_t>(t));
         g.rho_plane = (record && t >= t0 && t <= t1) ? a->d_rho_plane + (t - t0) * plane : nullptr;
-        adj::k_soft_step<S, R><<<grid, block, 0, a->stream>>>(g);
-        CULBM_CUDA(cudaGetLastError());
+        CULBM_CUDA(launch_step(t > t_begin, grid, block, a->stream, adj::k_soft_step<S, R>, g));
         cur = dst;
     }
     if (record && t_end >= t0 && t_end <= t1) {
@@ -917,8 +918,7 @@ culbm_status adjoint_segment(culbm_adj* a, int tb, int te, S* start, adj::Args<S
         const bool in_win = t >= t0 && t <= t1;
         g.obj_in = in_win ? obj_in : R(0);
         g.obj_out = in_win ? obj_out : R(0);
-        adj::k_adj_step<S, R><<<gr, block, 0, a->stream>>>(g, L);
-        CULBM_CUDA(cudaGetLastError());
+        CULBM_CUDA(launch_step(t < te - 1, gr, block, a->stream, adj::k_adj_step<S, R>, g, L));
         cur = 1 - cur;
     }
     adjms += elapsed(a);

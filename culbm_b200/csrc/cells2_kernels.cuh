@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_pull_cells2(const __grid_constant__ StepArgs<S, float> a, FastDiv row, int z0, f32x2 nzero)
 {
     const Domain& D = a.dom;
+    step_enter();
     const uint32_t t = 2 * (blockIdx.x * kCells2Threads + threadIdx.x);   // cell 0 within the plane
     if (t >= static_cast<uint32_t>(D.nxy)) return;
     const Pair c = pair_at(D, row, static_cast<int>(t), z0 + static_cast<int>(blockIdx.y));
@@ -371,6 +372,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_aa_odd_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
 {
     const Domain& D = a.dom;
+    step_enter();
     const int role = cells2_role(g);
     if (role >= 0) {
         CellCoord c;
@@ -434,6 +436,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_aa_even_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
 {
     const Domain& D = a.dom;
+    step_enter();
     const int role = cells2_role(g);
     if (role >= 0) {
         CellCoord c;

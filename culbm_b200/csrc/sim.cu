@@ -397,54 +397,51 @@ bool two_cells(const Domain& D)
     return Is16<S>::value && D.nx % 2 == 0;
 }
 
-// One pull step of the planes [za, zb) in the arguments' buffers.
+// One pull step of the planes [za, zb) in the arguments' buffers; `follows`:
+// the launch before it on the stream is a step of the same call.
 template <typename S, typename R>
-culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t st)
+culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t st, bool follows = false)
 {
     const Domain& D = a.dom;
-    bool done = false;
     if constexpr (Is16<S>::value) {
         if (two_cells<S>(D)) {
             FastDiv row;
             row.set(static_cast<uint32_t>(D.nx));
             const long long per_block = 2ll * kCells2Threads;
             const dim3 g(static_cast<unsigned>((D.nxy + per_block - 1) / per_block), zb - za);
-            k_pull_cells2<S><<<g, kCells2Threads, 0, st>>>(a, row, za, kNegZero2);
-            done = true;
+            CULBM_CUDA(launch_step(follows, g, kCells2Threads, st, k_pull_cells2<S>, a, row, za, kNegZero2));
+            return CULBM_OK;
         }
     }
-    if (!done)
-        k_pull_step<S, R><<<dim3((D.nx + 31) / 32, (D.ny + 7) / 8, zb - za), cell_block(), 0, st>>>(a, za);
-    CULBM_CUDA(cudaGetLastError());
+    const dim3 g((D.nx + 31) / 32, (D.ny + 7) / 8, zb - za);
+    CULBM_CUDA(launch_step(follows, g, cell_block(), st, k_pull_step<S, R>, a, za));
     return CULBM_OK;
 }
 
 // One in-place step of the planes [za, zb) (odd: layout A -> B).
 template <typename S, typename R>
-culbm_status launch_inplace(const StepArgs<S, R>& a, bool odd, int za, int zb, cudaStream_t st)
+culbm_status launch_inplace(const StepArgs<S, R>& a, bool odd, int za, int zb, cudaStream_t st, bool follows = false)
 {
     const Domain& D = a.dom;
-    bool done = false;
     if constexpr (Is16<S>::value) {
         if (two_cells<S>(D)) {
             long long blocks = 0;
             const Cells2Grid g = cells2_grid(D, za, zb, &blocks);
-            if (odd) k_aa_odd_cells2<S><<<static_cast<unsigned>(blocks), kCells2Threads, 0, st>>>(a, g, kNegZero2);
-            else k_aa_even_cells2<S><<<static_cast<unsigned>(blocks), kCells2Threads, 0, st>>>(a, g, kNegZero2);
-            done = true;
+            auto kern = odd ? k_aa_odd_cells2<S> : k_aa_even_cells2<S>;
+            CULBM_CUDA(launch_step(follows, static_cast<unsigned>(blocks), kCells2Threads, st, kern, a, g, kNegZero2));
+            return CULBM_OK;
         }
     }
-    if (!done && za == 0 && zb == D.nz) {
+    if (za == 0 && zb == D.nz) {
         const dim3 g = split_grid(D, AaShape<S>::rows, AaShape<S>::cols);
-        if (odd) k_aa_odd<S, R><<<g, aa_block<S>(), 0, st>>>(a);
-        else k_aa_even<S, R><<<g, aa_block<S>(), 0, st>>>(a);
-    } else if (!done) {
+        auto kern = odd ? k_aa_odd<S, R> : k_aa_even<S, R>;
+        CULBM_CUDA(launch_step(follows, g, aa_block<S>(), st, kern, a));
+    } else {
         const SlabSplit q = slab_split(D, za, zb, AaShape<S>::rows);
         const dim3 g = slab_split_grid(D, q, AaShape<S>::rows, AaShape<S>::cols);
-        if (odd) k_aa_odd_slab<S, R><<<g, aa_block<S>(), 0, st>>>(a, q);
-        else k_aa_even_slab<S, R><<<g, aa_block<S>(), 0, st>>>(a, q);
+        auto kern = odd ? k_aa_odd_slab<S, R> : k_aa_even_slab<S, R>;
+        CULBM_CUDA(launch_step(false, g, aa_block<S>(), st, kern, a, q));
     }
-    CULBM_CUDA(cudaGetLastError());
     return CULBM_OK;
 }
 
@@ -512,12 +509,12 @@ culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
         if (!s->inplace) {
             auto a = make_args<S>(s, s->cur, 1 - s->cur);
             a.seed = seed;
-            CULBM_TRY((launch_pull<S, R>(a, 0, s->dom.nz, s->stream)));
+            CULBM_TRY((launch_pull<S, R>(a, 0, s->dom.nz, s->stream, k > 0)));
             s->cur ^= 1;
         } else {
             auto a = make_args<S>(s, 0, 0);
             a.seed = seed;
-            CULBM_TRY((launch_inplace<S, R>(a, s->aa_phase == 0, 0, s->dom.nz, s->stream)));
+            CULBM_TRY((launch_inplace<S, R>(a, s->aa_phase == 0, 0, s->dom.nz, s->stream, k > 0)));
             s->aa_phase ^= 1;
         }
         s->launches += 1;

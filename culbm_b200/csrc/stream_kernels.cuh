@@ -226,6 +226,34 @@ __device__ __forceinline__ void load_pulled(const StepArgs<S, R>& a, int x, int 
     }
 }
 
+// Programmatic dependent launch: consecutive steps are launched with
+// programmatic stream serialisation (launch_step), so the next step's blocks
+// may start while this grid's last blocks run.  Each step lets its dependents
+// start at once and waits for the previous grid (complete, its memory
+// visible) before touching memory; the wait is the hardware's own and always
+// ends.  Launched the ordinary way, both instructions do nothing.
+__device__ __forceinline__ void step_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A step launch; `follows`: the launch before it on the stream is a step too.
+template <typename... P, typename... A>
+cudaError_t launch_step(bool follows, dim3 grid, dim3 block, cudaStream_t st, void (*kernel)(P...), const A&... args)
+{
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = follows ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, kernel, args...);
+}
+
 struct CellCoord {
     int x, y, z, i;
     bool valid;
@@ -269,6 +297,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
     k_pull_step(const __grid_constant__ StepArgs<S, R> a, int z0)
 {
     const CellCoord c = cell_of_thread(a.dom, z0);
+    step_enter();
     if (c.valid) pull_cell<S, R>(a, c);
 }
 
@@ -591,6 +620,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_aa_odd(const __
 {
     CellCoord c;
     const int kind = split_cell(a.dom, 0, c);
+    step_enter();
     if (kind == ROWS_OUTER)
         aa_odd_cell<S, R, ROWS_OUTER>(a, c);
     else if (kind == ROWS_INNER)
@@ -602,6 +632,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_aa_even(const _
 {
     CellCoord c;
     const int kind = split_cell(a.dom, 0, c);
+    step_enter();
     if (kind == ROWS_OUTER)
         aa_even_cell<S, R, ROWS_OUTER>(a, c);
     else if (kind == ROWS_INNER)

@@ -132,17 +132,6 @@ __device__ __forceinline__ bool in_tile(int px, int py, int pz, int bx, int by, 
 // registers) spill 36-140 bytes.
 constexpr int kTileMinBlocks = 4;
 
-// Programmatic dependent launch: the tile steps of a round are launched
-// with programmatic stream serialisation, so the next step's blocks may start
-// while this grid's last blocks run.  Each step lets its dependents start at
-// once and waits for the previous grid (complete, its memory visible) before
-// touching memory; the wait is the hardware's own and always ends.
-__device__ __forceinline__ void tile_step_enter()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Pull of all 27 populations from the global state with the domain clamp.
 template <typename S, typename R, bool HINT>
 __device__ __forceinline__ void tile_pull_global(const TileArgs<S, R>& a, const TileCell& c, int sel, int offz, R* f)
@@ -233,7 +222,7 @@ __device__ __forceinline__ void tile_file_clamp_sources(const TileArgs<S, R>& a,
 template <typename S, typename R, bool ONE, bool HINT>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_first(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active) return;
     const int ring = a.g.ring_nz;
@@ -260,7 +249,7 @@ __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_first(const __g
 template <typename S, typename R>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_odd(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active) return;
     const Domain& D = a.dom;
@@ -310,7 +299,7 @@ __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_odd(const __gri
 template <typename S, typename R>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_even(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active) return;
     const uint8_t op = a.ops[c.gi];
@@ -331,7 +320,7 @@ __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_even(const __gr
 template <int LAYOUT, typename S, typename R, bool HINT>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_aa_last(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active || !c.correct) return;
     const uint8_t op = a.ops[c.gi];
@@ -384,7 +373,7 @@ __device__ __forceinline__ void tile_pull(const TileArgs<S, R>& a, const Pops<S>
 template <typename S, typename R, bool ONE, bool HINT>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_pull_first(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active) return;
     const int ring = a.g.ring_nz;
@@ -409,7 +398,7 @@ __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_pull_first(const _
 template <typename S, typename R>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_pull_mid(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active) return;
     const uint8_t op = a.ops[c.gi];
@@ -428,7 +417,7 @@ __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_pull_mid(const __g
 template <typename S, typename R, bool HINT>
 __global__ void __launch_bounds__(256, kTileMinBlocks) k_tile_pull_last(const __grid_constant__ TileArgs<S, R> a)
 {
-    tile_step_enter();
+    step_enter();
     const TileCell c = tile_cell(a);
     if (!c.active || !c.correct) return;
     const uint8_t op = a.ops[c.gi];
