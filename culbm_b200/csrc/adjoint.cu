@@ -88,12 +88,13 @@ __device__ __forceinline__ void pull_state(const Args<S, R>& a, int x, int y, in
 }
 
 // Boundary handling and soft collision of the forward model (in place on f).
-template <typename R>
+// E > 0: f holds raw values 2^E f in and out (same bits after unscaling).
+template <typename R, int E>
 __device__ __forceinline__ void soft_update(uint8_t op, R inv_tau, R s, const float* rho, const float* vx,
                                             const float* vy, const float* vz, int i, R* f)
 {
     using A = Rn<R>;
-    if (op & OP_EQU) equilibrium<R>(R(rho[i]), R(vx[i]), R(vy[i]), R(vz[i]), f);
+    if (op & OP_EQU) equilibrium<R, E>(R(rho[i]), R(vx[i]), R(vy[i]), R(vz[i]), f);
     if (op & OP_BB) {
 #pragma unroll
         for (int d = 0; d < 13; ++d) {
@@ -104,9 +105,9 @@ __device__ __forceinline__ void soft_update(uint8_t op, R inv_tau, R s, const fl
     }
     if (!(op & OP_COLLIDE)) return;
     R r, ux, uy, uz;
-    moments(f, r, ux, uy, uz);
+    moments<R, E>(f, r, ux, uy, uz);
     EquTerms<R> t;
-    equ_terms(r, ux, uy, uz, t);
+    equ_terms<R, E>(r, ux, uy, uz, t);
     const R om = A::sub(R(1), inv_tau);
     const bool soft = s != R(0);
 #pragma unroll
@@ -128,11 +129,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_soft_step(const
     const CellCoord c = cell_of_thread(a.dom);
     step_enter();
     if (!c.valid) return;
+    constexpr int E = ScaleExp<S>::value;
     const uint8_t op = a.ops[c.i];
+    const R soft = R(a.soft[c.i]);
     R f[27];
-    if (op & OP_LOAD) {
-        pull_state(a, c.x, c.y, c.z, c.i, f);
-    } else {
+    pull_state<ROWS_OUTER, true>(a, c.x, c.y, c.z, c.i, f);   // before the op byte is looked at
+    if (!(op & OP_LOAD)) {
 #pragma unroll
         for (int d = 0; d < 27; ++d) f[d] = R(0);
     }
@@ -141,19 +143,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_soft_step(const
         double r = 0.0;
         if (op & OP_COLLIDE) {
             R rr, ux, uy, uz;
-            moments(f, rr, ux, uy, uz);
+            moments<R, E>(f, rr, ux, uy, uz);
             r = static_cast<double>(rr);
         }
         const int q = c.y + a.dom.ny * c.z;
         if (c.x == a.plane_in) a.rho_plane[q] = r;
         if (c.x == a.plane_out) a.rho_plane[a.dom.ny * a.dom.nz + q] = r;
     }
-    soft_update<R>(op, a.inv_tau, R(a.soft[c.i]), a.rho, a.vx, a.vy, a.vz, c.i, f);
-    if (op & OP_STORE) {
-        const uint32_t hc = cell_hash(static_cast<uint32_t>(c.i), a.seed);
-#pragma unroll
-        for (int d = 0; d < 27; ++d) put(a.dst.p[d] + c.i, f[d], hc, d);
-    }
+    soft_update<R, E>(op, a.inv_tau, soft, a.rho, a.vx, a.vy, a.vz, c.i, f);
+    if (op & OP_STORE)
+        put27_raw<S>(f, cell_hash(static_cast<uint32_t>(c.i), a.seed), [&](int d) { return a.dst.p[d] + c.i; });
 }
 
 // rho of the pulled state on the two measurement planes (the last state of
@@ -246,16 +245,17 @@ __device__ __forceinline__ void feq_vjp(const R* l, R ux, R uy, R uz, R& a_rho, 
     bz = R(3) * Lz + R(9) * Lccz - R(3) * uz * L0;
 }
 
-// FP64 warp sum of v added to the warp's own accumulator slots[warp] (no
-// atomics and no block barrier: each warp owns its slot, so the result does
-// not depend on scheduling, and a warp leaves as soon as it is done).  All
-// 32 lanes must arrive.
+// FP64 warp sum of v added to the warp's own accumulator slots[warp].  Each
+// warp owns its slot, so the result does not depend on scheduling; the add is
+// an atomic only to be done in L2, so that the warp does not wait for the old
+// value.  No block barrier: a warp leaves as soon as it is done.  All 32
+// lanes must arrive.
 __device__ __forceinline__ void warp_accumulate(double v, double* slots)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
     const int t = threadIdx.x + blockDim.x * threadIdx.y;
-    if ((t & 31) == 0) slots[t >> 5] += v;
+    if ((t & 31) == 0) atomicAdd(slots + (t >> 5), v);
 }
 
 // Adjoint of the stored population d of cell c: the sum of nu_d over the
@@ -484,7 +484,7 @@ __device__ __forceinline__ void adj_cell(const Args<S, R>& a, const CellCoord c,
     if (ROWS == ROWS_INNER && xw != 0 && xw + 31 < D.nx - 1) {
         for_dirs([&](auto dd) {
             constexpr int d = decltype(dd)::value;
-            l[d] = a.nu_in[d][c.i + nb_off(D, d)];
+            l[d] = ld_stream_raw<R, R>(a.nu_in[d] + (c.i + nb_off(D, d)));
         });
         for_dirs([&](auto dd) {
             constexpr int d = decltype(dd)::value;
@@ -521,7 +521,7 @@ __device__ __forceinline__ void adj_cell(const Args<S, R>& a, const CellCoord c,
     m.finish(fscale, (op & OP_BB) != 0, rho, ux, uy, uz);
     reverse_cell(op, a.inv_tau, s, fscale, dots, rho, ux, uy, uz, l, gs, gw);
     if (!equ && (op & OP_COLLIDE) && store) {
-        a.g_soft[c.i] += static_cast<double>(gs);
+        atomicAdd(a.g_soft + c.i, static_cast<double>(gs));   // the cell's only add of the step, done in L2
         gtau_local = static_cast<double>(gw);
     }
     const bool pulls = load && store && !equ;
