@@ -95,8 +95,8 @@ class AdjointProblem:
     def gradient(self):
         """(J, dJ/dinvTau, dJ/ds [N], dJ/d(rho, vx, vy, vz) of the EQU inputs [4, N])."""
         j, gt = C.c_double(), C.c_double()
-        gs = np.zeros(self.n, np.float64)
-        gm = np.zeros(4 * self.n, np.float64)
+        gs = np.empty(self.n, np.float64)
+        gm = np.empty(4 * self.n, np.float64)
         check(lib().culbm_adj_gradient(self._h, C.byref(j), C.byref(gt), _ptr(gs), _ptr(gm)))
         return j.value, gt.value, gs, gm.reshape(4, self.n)
 

@@ -31,6 +31,8 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "sim_internal.cuh"
@@ -54,7 +56,7 @@ struct Args {
     R* nu_out[27];    // adjoint: nu^t
     double* g_soft;
     double* g_tau;
-    double* g_mac[4];
+    double* g_mac[4];   // by position in equ_cells
     int plane_in, plane_out;
     R obj_in, obj_out;   // dJ/df_d of one in/out plane cell at this time (0 outside the window)
     uint32_t seed;
@@ -536,14 +538,15 @@ __device__ __forceinline__ void adj_cell(const Args<S, R>& a, const CellCoord c,
     for (int d = 0; d < 27; ++d) a.nu_out[d][c.i] = l[d];
 }
 
-// The EQU cell i of one adjoint step: f1 = feq(rho_in, u_in), the gather
+// The EQU cell i = equ_cells[k] of one adjoint step: f1 = feq(rho_in, u_in), the gather
 // with the general clamp rule, the reverse of bounce-back and collision, and
 // dJ/d(rho_in, u_in) from d feq / d(rho, u).  Its nu (no pull, so dJ/df
 // only) is written by adj_cell.
 template <typename S, typename R>
-__device__ __forceinline__ void adj_equ_cell(const Args<S, R>& a, int i, double& gtau_local)
+__device__ __forceinline__ void adj_equ_cell(const Args<S, R>& a, int k, double& gtau_local)
 {
     const Domain& D = a.dom;
+    const int i = a.equ_cells[k];
     CellCoord c;
     c.i = i;
     c.x = i % D.nx;
@@ -578,10 +581,10 @@ __device__ __forceinline__ void adj_equ_cell(const Args<S, R>& a, int i, double&
     }
     R ar, bx, by, bz;
     feq_vjp(l, vx, vy, vz, ar, bx, by, bz);
-    a.g_mac[0][i] += static_cast<double>(ar);
-    a.g_mac[1][i] += static_cast<double>(r_in * bx);
-    a.g_mac[2][i] += static_cast<double>(r_in * by);
-    a.g_mac[3][i] += static_cast<double>(r_in * bz);
+    a.g_mac[0][k] += static_cast<double>(ar);
+    a.g_mac[1][k] += static_cast<double>(r_in * bx);
+    a.g_mac[2][k] += static_cast<double>(r_in * by);
+    a.g_mac[3][k] += static_cast<double>(r_in * bz);
 }
 
 // Grid of one adjoint-step launch: equ_z grid-z slices of blocks that take
@@ -615,7 +618,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
     if (static_cast<int>(blockIdx.z) < L.equ_z) {
         const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
         const int k = blk * 256 + threadIdx.x + 32 * threadIdx.y;
-        if (k < a.n_equ) adj_equ_cell(a, a.equ_cells[k], gtau_local);
+        if (k < a.n_equ) adj_equ_cell(a, k, gtau_local);
     } else {
         CellCoord c;
         const int kind = split_cell(a.dom, L.equ_z, c);
@@ -675,17 +678,19 @@ struct culbm_adj {
     void* d_nu = nullptr;       // 2 x 27 N of the arithmetic type
     double* d_gsoft = nullptr;
     double* d_gtau = nullptr;
-    double* d_gmac = nullptr;   // 4 N
+    double* d_gmac = nullptr;   // 4 n_equ
     double* d_psum = nullptr;   // 2 per time step of the window
     double* d_rho_plane = nullptr;  // window x 2 planes x ny*nz
     long long n_tau_blocks = 0;     // warps of one adjoint-step launch (one FP64 slot each)
     long long tau_capacity = 0;
     int* d_equ = nullptr;           // EQU cells, increasing
-    int n_equ = 0, equ_capacity = 0;
+    int n_equ = 0, equ_capacity = 0, gmac_capacity = 0;
     int n_in = 0, n_out = 0;
     uint64_t device_bytes = 0;
     float t_fwd = 0, t_rec = 0, t_adj = 0;
-    std::vector<uint32_t> h_flag;
+    std::vector<int> h_equ;         // the EQU cells on the host
+    std::vector<cudaEvent_t> marks; // events of one gradient, in stream order (kept for the next)
+    std::vector<int> mark_of;       // what the time up to each mark was spent on
 };
 
 namespace {
@@ -727,6 +732,7 @@ void adj_release(culbm_adj* a)
     cudaFree(a->d_rho_plane);
     for (auto& e : a->ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : a->marks) cudaEventDestroy(e);
     if (a->stream) cudaStreamDestroy(a->stream);
     delete a;
 }
@@ -767,7 +773,7 @@ adj::Args<S, typename ArithOf<S>::type> base_args(culbm_adj* a)
     g.inv_tau = static_cast<R>(a->inv_tau);
     g.g_soft = a->d_gsoft;
     g.g_tau = a->d_gtau;
-    for (int k = 0; k < 4; ++k) g.g_mac[k] = a->d_gmac + k * a->n;
+    for (int k = 0; k < 4; ++k) g.g_mac[k] = a->d_gmac + k * static_cast<long long>(a->n_equ);
     g.plane_in = a->cfg.plane_x[0];
     g.plane_out = a->cfg.plane_x[1];
     return g;
@@ -841,6 +847,39 @@ float elapsed(culbm_adj* a)
     return ms;
 }
 
+// Phases of a gradient: the time from one mark to the next is spent on the
+// later one's phase.  Read once at the end, so that the segments follow one
+// another without the host waiting in between.
+enum Phase { PHASE_NONE, PHASE_FORWARD, PHASE_RECOMPUTE, PHASE_ADJOINT };
+
+culbm_status mark(culbm_adj* a, Phase p)
+{
+    const size_t k = a->mark_of.size();
+    if (k == a->marks.size()) {
+        cudaEvent_t e = nullptr;
+        CULBM_CUDA(cudaEventCreate(&e));
+        a->marks.push_back(e);
+    }
+    CULBM_CUDA(cudaEventRecord(a->marks[k], a->stream));
+    a->mark_of.push_back(p);
+    return CULBM_OK;
+}
+
+culbm_status read_marks(culbm_adj* a)
+{
+    float t[4] = {0, 0, 0, 0};
+    CULBM_CUDA(cudaStreamSynchronize(a->stream));
+    for (size_t k = 1; k < a->mark_of.size(); ++k) {
+        float ms = 0;
+        CULBM_CUDA(cudaEventElapsedTime(&ms, a->marks[k - 1], a->marks[k]));
+        t[a->mark_of[k]] += ms;
+    }
+    a->t_fwd = t[PHASE_FORWARD];
+    a->t_rec = t[PHASE_RECOMPUTE];
+    a->t_adj = t[PHASE_ADJOINT];
+    return CULBM_OK;
+}
+
 template <typename S>
 culbm_status run_forward(culbm_adj* a, bool checkpoints)
 {
@@ -894,8 +933,7 @@ culbm_status run_forward_mixed(culbm_adj* a, bool checkpoints)
 // te-1 .. tb.
 template <typename S>
 culbm_status adjoint_segment(culbm_adj* a, int tb, int te, S* start, adj::Args<S, typename ArithOf<S>::type>& g,
-                             typename ArithOf<S>::type* const nu[2], int& cur, float& rec, float& adjms,
-                             bool states_present = false)
+                             typename ArithOf<S>::type* const nu[2], int& cur, bool states_present = false)
 {
     using R = typename ArithOf<S>::type;
     const int t0 = a->cfg.window[0], t1 = a->cfg.window[1];
@@ -907,7 +945,7 @@ culbm_status adjoint_segment(culbm_adj* a, int tb, int te, S* start, adj::Args<S
     const dim3 gr = adj::adj_grid(a->dom, a->n_equ);
     auto slot_of = [&](int t) -> S* { return state_ptr<S>(a, SEG, t - tb - 1); };
     if (!states_present) CULBM_TRY(forward_run<S>(a, tb, te - 1, start, slot_of, false));
-    rec += elapsed(a);
+    CULBM_TRY(mark(a, PHASE_RECOMPUTE));
     for (int t = te - 1; t >= tb; --t) {
         S* st = (t == tb) ? start : state_ptr<S>(a, SEG, t - tb - 1);
         set_pops<S, R>(g.src, st, a->n);
@@ -921,8 +959,7 @@ culbm_status adjoint_segment(culbm_adj* a, int tb, int te, S* start, adj::Args<S
         CULBM_CUDA(launch_step(t < te - 1, gr, block, a->stream, adj::k_adj_step<S, R>, g, L));
         cur = 1 - cur;
     }
-    adjms += elapsed(a);
-    return CULBM_OK;
+    return mark(a, PHASE_ADJOINT);
 }
 
 template <typename S>
@@ -934,17 +971,18 @@ culbm_status run_gradient(culbm_adj* a)
     const double nT = t1 - t0 + 1;
     const dim3 grid = cell_grid(a->dom), block = cell_block();
 
-    CULBM_CUDA(cudaEventRecord(a->ev[0], a->stream));
+    a->mark_of.clear();
+    CULBM_TRY(mark(a, PHASE_NONE));
     if (a->mixed) {
         CULBM_TRY(run_forward_mixed<S>(a, true));
     } else {
         CULBM_TRY(run_forward<S>(a, true));
     }
-    a->t_fwd = elapsed(a);
+    CULBM_TRY(mark(a, PHASE_FORWARD));
 
     CULBM_CUDA(cudaMemsetAsync(a->d_gsoft, 0, a->n * sizeof(double), a->stream));
     CULBM_CUDA(cudaMemsetAsync(a->d_gtau, 0, a->n_tau_blocks * sizeof(double), a->stream));
-    CULBM_CUDA(cudaMemsetAsync(a->d_gmac, 0, 4 * a->n * sizeof(double), a->stream));
+    if (a->n_equ) CULBM_CUDA(cudaMemsetAsync(a->d_gmac, 0, 4ull * a->n_equ * sizeof(double), a->stream));
     R* const nu[2] = {static_cast<R*>(a->d_nu), static_cast<R*>(a->d_nu) + 27 * a->n};
     auto g = base_args<S>(a);
     g.g_tau_block = a->d_gtau;
@@ -958,8 +996,7 @@ culbm_status run_gradient(culbm_adj* a)
         adj::k_adj_init<S, R><<<grid, block, 0, a->stream>>>(g);
         CULBM_CUDA(cudaGetLastError());
     }
-    float rec = 0, adjms = 0;
-    CULBM_CUDA(cudaEventRecord(a->ev[0], a->stream));
+    CULBM_TRY(mark(a, PHASE_NONE));
     for (int k = (T - 1) / K; k >= 0; --k) {
         const int tb = k * K, te = std::min(T, (k + 1) * K);
         S* ck = state_ptr<S>(a, CKPT, k);
@@ -967,7 +1004,7 @@ culbm_status run_gradient(culbm_adj* a)
             // the forward pass left the last segment's states in place
             // (not in the mixed mode, whose forward states are FP32)
             const bool last = !a->mixed && k == (T - 1) / K;
-            CULBM_TRY(adjoint_segment<S>(a, tb, te, ck, g, nu, cur, rec, adjms, last));
+            CULBM_TRY(adjoint_segment<S>(a, tb, te, ck, g, nu, cur, last));
             continue;
         }
         // two levels: one pass over the outer segment stores F^{tb + j K2},
@@ -979,18 +1016,42 @@ culbm_status run_gradient(culbm_adj* a)
                 return r % K2 == 0 ? state_ptr<S>(a, INNER, r / K2 - 1) : state_ptr<S>(a, SEG, t & 1);
             };
             CULBM_TRY(forward_run<S>(a, tb, tb + nin * K2, ck, slot_of, false));
-            rec += elapsed(a);
+            CULBM_TRY(mark(a, PHASE_RECOMPUTE));
         }
         for (int j = nin; j >= 0; --j) {
             const int sb = tb + j * K2, se = std::min(te, sb + K2);
             S* start = j ? state_ptr<S>(a, INNER, j - 1) : ck;
-            CULBM_TRY(adjoint_segment<S>(a, sb, se, start, g, nu, cur, rec, adjms));
+            CULBM_TRY(adjoint_segment<S>(a, sb, se, start, g, nu, cur));
         }
     }
-    a->t_rec = rec;
-    a->t_adj = adjms;
     return CULBM_OK;
 }
+
+// Fills two host arrays with zeros on a thread of its own (here if no thread
+// can be had); joined before it goes out of scope.
+class ZeroFill {
+public:
+    void start(double* p, size_t np, double* q, size_t nq)
+    {
+        auto fill = [=] {
+            if (p) std::memset(p, 0, np * sizeof(double));
+            if (q) std::memset(q, 0, nq * sizeof(double));
+        };
+        try {
+            t_ = std::thread(fill);
+        } catch (const std::system_error&) {
+            fill();
+        }
+    }
+    void wait()
+    {
+        if (t_.joinable()) t_.join();
+    }
+    ~ZeroFill() { wait(); }
+
+private:
+    std::thread t_;
+};
 
 // Checkpoint plan: outer stride K, inner stride K2 (0: one level) and the
 // number of full states each needs.
@@ -1165,8 +1226,6 @@ culbm_status culbm_adj_create(const culbm_adj_config* cfg, culbm_adj** out)
         CULBM_TRY(adj_alloc(a, &a->d_nu, 2ull * 27 * n * a->rsize, "adjoint populations"));
         CULBM_TRY(adj_alloc(a, &p, n * sizeof(double), "soft gradient"));
         a->d_gsoft = static_cast<double*>(p);
-        CULBM_TRY(adj_alloc(a, &p, 4 * n * sizeof(double), "EQU input gradients"));
-        a->d_gmac = static_cast<double*>(p);
         const long long nt = c.window[1] - c.window[0] + 1;
         CULBM_TRY(adj_alloc(a, &p, 2ull * nt * sizeof(double), "objective sums"));
         a->d_psum = static_cast<double*>(p);
@@ -1236,11 +1295,17 @@ culbm_status culbm_adj_set_state(culbm_adj* a, const uint32_t* flag, const float
         CULBM_CUDA(cudaFree(a->d_equ));
         a->d_equ = nullptr;
         a->device_bytes -= a->equ_capacity * sizeof(int);
-        a->equ_capacity = 0;
+        CULBM_CUDA(cudaFree(a->d_gmac));
+        a->d_gmac = nullptr;
+        a->device_bytes -= a->gmac_capacity * 4 * sizeof(double);
+        a->equ_capacity = a->gmac_capacity = 0;
         void* p = nullptr;
         CULBM_TRY(adj_alloc(a, &p, n_equ * sizeof(int), "EQU cell list"));
         a->d_equ = static_cast<int*>(p);
         a->equ_capacity = n_equ;
+        CULBM_TRY(adj_alloc(a, &p, 4ull * n_equ * sizeof(double), "EQU input gradients"));
+        a->d_gmac = static_cast<double*>(p);
+        a->gmac_capacity = n_equ;
     }
     {
         const dim3 gr = adj::adj_grid(a->dom, n_equ);
@@ -1260,6 +1325,7 @@ culbm_status culbm_adj_set_state(culbm_adj* a, const uint32_t* flag, const float
         a->n_tau_blocks = slots;
     }
     a->n_equ = n_equ;
+    a->h_equ = equ;
     if (n_equ)
         CULBM_CUDA(cudaMemcpyAsync(a->d_equ, equ.data(), n_equ * sizeof(int), cudaMemcpyHostToDevice, a->stream));
     CULBM_CUDA(cudaMemcpyAsync(a->d_ops, ops.data(), n, cudaMemcpyHostToDevice, a->stream));
@@ -1312,11 +1378,19 @@ culbm_status culbm_adj_gradient(culbm_adj* a, double* J, double* dJ_dinv_tau, do
 {
     if (!a) return fail(CULBM_ERR_INVALID_ARGUMENT, "adjoint handle is NULL");
     CULBM_CUDA(cudaSetDevice(a->dev));
+    const size_t n = static_cast<size_t>(a->n);
+    // dJ/d(rho, u) is zero but at the EQU cells: only their values leave the
+    // device, and the zeros are written here while it computes (dJ/ds too,
+    // so that its copy meets mapped pages).  192x136x140: 28 -> 3 ms of the
+    // call spent on its outputs and on waits between segments.
+    ZeroFill zero;
+    zero.start(dJ_dsoft, n, dJ_dmac, 4 * n);
     CULBM_TRY(adj_with_storage(a, [&](auto tag) { return run_gradient<typename decltype(tag)::type>(a); }));
+    CULBM_TRY(read_marks(a));
     double j = 0;
     CULBM_TRY(objective(a, &j));
     if (J) *J = j;
-    const size_t n = static_cast<size_t>(a->n);
+    zero.wait();
     if (dJ_dinv_tau) {
         std::vector<double> g(static_cast<size_t>(a->n_tau_blocks));
         CULBM_CUDA(cudaMemcpy(g.data(), a->d_gtau, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
@@ -1325,7 +1399,13 @@ culbm_status culbm_adj_gradient(culbm_adj* a, double* J, double* dJ_dinv_tau, do
         *dJ_dinv_tau = s;
     }
     if (dJ_dsoft) CULBM_CUDA(cudaMemcpy(dJ_dsoft, a->d_gsoft, n * sizeof(double), cudaMemcpyDeviceToHost));
-    if (dJ_dmac) CULBM_CUDA(cudaMemcpy(dJ_dmac, a->d_gmac, 4 * n * sizeof(double), cudaMemcpyDeviceToHost));
+    if (dJ_dmac && a->n_equ) {
+        const size_t m = static_cast<size_t>(a->n_equ);
+        std::vector<double> g(4 * m);
+        CULBM_CUDA(cudaMemcpy(g.data(), a->d_gmac, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
+        for (size_t k = 0; k < 4; ++k)
+            for (size_t q = 0; q < m; ++q) dJ_dmac[k * n + a->h_equ[q]] = g[k * m + q];
+    }
     return CULBM_OK;
 }
 

@@ -237,3 +237,35 @@ def test_zero_soft_field_is_the_plain_step(culbm):
             if t < window[1]:
                 sim.step(1)
     assert abs(J - acc / (window[1] - window[0] + 1)) <= 1e-12 * abs(J)
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16sr"])
+def test_equ_cells_change_between_gradients(storage):
+    """The EQU list and its gradients live by list position on the device: one
+    handle over states with fewer, more and no EQU cells gives the bits of a
+    fresh handle, with zeros in dJ/d(rho, u) away from the EQU cells."""
+    dims = (34, 9, 7)
+    sc, f, r, ux, uy, uz, soft = case(*dims, bumps=2)
+    flags = [f.copy() for _ in range(3)]
+    extra = np.flatnonzero(f == S.FLUID)[::11]
+    flags[1][extra] = S.EQUILIBRIUM
+    flags[2][(f & S.EQU) != 0] = S.FLUID
+    flags[2].reshape(dims[::-1])[3, 4, 5] = S.EQUILIBRIUM
+    none = f.copy()
+    none[(f & S.EQU) != 0] = S.FLUID
+
+    def problem():
+        return AdjointProblem(dims, window=(6, 10), inv_tau=0.7, checkpoint_every=4, storage=storage)
+
+    with problem() as kept:
+        for fl in flags + [none, flags[1]]:
+            kept.set_state(fl, r, ux, uy, uz, soft)
+            got = kept.gradient()
+            with problem() as fresh:
+                fresh.set_state(fl, r, ux, uy, uz, soft)
+                want = fresh.gradient()
+            for a, b in zip(got, want):
+                assert np.array_equal(np.asarray(a), np.asarray(b))
+            assert not got[3][:, (fl & S.EQU) == 0].any()
+        info = kept.info()
+        assert info["forward_ms"] > 0 and info["recompute_ms"] > 0 and info["adjoint_ms"] > 0
