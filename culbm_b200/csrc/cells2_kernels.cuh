@@ -17,8 +17,8 @@
 // and other cells take the one-cell code after it.
 //
 // FP16-SR channel with spheres, 288x272x280: pull 585 -> 478 us per step
-// (45.9k MLUPS, 0.76 of the copy bandwidth), in place 666 -> 601 us; 512x512x256
-// 1744 -> 1428 us and 1948 -> 1736 us.  What bounds them now: latency (24 warps
+// (45.9k MLUPS, 0.76 of the copy bandwidth), in place 666 -> 596 us; 512x512x256
+// 1744 -> 1428 us and 1948 -> 1729 us.  What bounds them now: latency (24 warps
 // per SM, 53 % issue, loads waited for first) and, in place, instruction
 // fetches besides (face rows and inner rows are two large bodies of code).
 //
@@ -280,17 +280,16 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     other_cells(kind.p0 && packed, kind.p1 && packed, [&](int k) { pull_cell<S, float>(a, cell_in_pair(c, k)); });
 }
 
-// Launch of an in-place step over the planes of a SlabSplit: `faces` blocks
-// take the y/z-face rows one cell per thread (general clamp code), and
-// `blocks_per_plane` blocks per interior plane take the pairs of its inner
-// rows.  The face blocks wait on long chains of few instructions; every
-// `every`-th block of the launch is one, over its first four fifths, so that
-// they always share an SM with inner blocks and none starts at the end (2 %
-// faster than all of them first, at 288x272x280).
+// Launch of an in-place step over the planes of a SlabSplit: first `faces`
+// blocks that take the y/z-face rows one cell per thread (general clamp
+// code), then `blocks_per_plane` blocks per interior plane for the pairs of
+// its inner rows.  (Face blocks spread over the launch instead evict the inner
+// rows' code from the instruction caches: 66.6 against 64.5 us per FP16-SR
+// step at 160x120x100, 598 against 596 us at 288x272x280.)
 struct Cells2Grid {
     SlabSplit q;
-    FastDiv row, per_plane, step;
-    int faces, blocks_per_plane, every;
+    FastDiv row, per_plane;
+    int faces, blocks_per_plane;
 };
 
 inline Cells2Grid cells2_grid(const Domain& D, int za, int zb, long long* blocks)
@@ -301,21 +300,10 @@ inline Cells2Grid cells2_grid(const Domain& D, int za, int zb, long long* blocks
     const long long inner = D.ny > 2 ? 1ll * D.nx * (D.ny - 2) : 0;   // even
     g.faces = static_cast<int>((face + kCells2Threads - 1) / kCells2Threads);
     g.blocks_per_plane = static_cast<int>((inner + 2 * kCells2Threads - 1) / (2 * kCells2Threads));
-    const long long pairs = 1ll * g.blocks_per_plane * g.q.ni;
-    *blocks = g.faces + pairs;
-    g.every = static_cast<int>(g.faces ? std::max(1ll, *blocks * 4 / 5 / g.faces) : 1);
+    *blocks = g.faces + 1ll * g.blocks_per_plane * g.q.ni;
     g.row.set(static_cast<uint32_t>(D.nx));
     g.per_plane.set(static_cast<uint32_t>(std::max(g.blocks_per_plane, 1)));
-    g.step.set(static_cast<uint32_t>(g.every));
     return g;
-}
-
-// Role of this block: the face block's number, or -1 - (inner block's number).
-__device__ __forceinline__ int cells2_role(const Cells2Grid& g)
-{
-    const int b = static_cast<int>(blockIdx.x), k = static_cast<int>(g.step.div(blockIdx.x));
-    if (k >= g.faces) return -1 - (b - g.faces);
-    return b == k * g.every ? k : -1 - (b - k - 1);
 }
 
 // Face-row cell t of a launch (0-based over the slab's z-face planes, then
@@ -373,14 +361,13 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
 {
     const Domain& D = a.dom;
     step_enter();
-    const int role = cells2_role(g);
-    if (role >= 0) {
+    if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
         CellCoord c;
-        if (face_cell(D, g, role * kCells2Threads + threadIdx.x, c)) aa_odd_cell<S, float, ROWS_OUTER>(a, c);
+        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_odd_cell<S, float, ROWS_OUTER>(a, c);
         return;
     }
     Pair c;
-    if (!inner_pair(D, g, static_cast<uint32_t>(-1 - role), c)) return;
+    if (!inner_pair(D, g, blockIdx.x - static_cast<uint32_t>(g.faces), c)) return;
     const uint32_t ops = ops_of(a.ops, c.i);
     uint32_t w[27];   // loaded before the op bytes are looked at
 #pragma unroll
@@ -437,14 +424,13 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
 {
     const Domain& D = a.dom;
     step_enter();
-    const int role = cells2_role(g);
-    if (role >= 0) {
+    if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
         CellCoord c;
-        if (face_cell(D, g, role * kCells2Threads + threadIdx.x, c)) aa_even_cell<S, float, ROWS_OUTER>(a, c);
+        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_even_cell<S, float, ROWS_OUTER>(a, c);
         return;
     }
     Pair c;
-    if (!inner_pair(D, g, static_cast<uint32_t>(-1 - role), c)) return;
+    if (!inner_pair(D, g, blockIdx.x - static_cast<uint32_t>(g.faces), c)) return;
     const uint32_t ops = ops_of(a.ops, c.i);
     uint32_t w[27];   // loaded before the op bytes are looked at
 #pragma unroll
