@@ -385,6 +385,33 @@ __device__ __forceinline__ void put27_raw_if(const R* f, uint32_t hcell, A&& add
     }
 }
 
+// The 27 raw values of one cell as the 16-bit patterns put27_raw stores,
+// directions k and 26 - k in one word: half the registers of the values, where
+// they are stored more than once.
+template <typename S>
+struct Bits27 {
+    uint32_t w[14];
+    __device__ __forceinline__ Bits27(const float* f, uint32_t hcell)
+    {
+#pragma unroll
+        for (int k = 0; k < 13; ++k) w[k] = Pack2<S>::cvt(f[26 - k], f[k], IsSR<S>::value ? sr_word_pair(hcell, k) : 0u);
+        w[13] = enc16_raw<S>(f[13], hcell, 13);
+    }
+    __device__ __forceinline__ unsigned short at(int d) const
+    {
+        return static_cast<unsigned short>(d <= 13 ? w[d] : w[26 - d] >> 16);
+    }
+    // at(d) where d is not known at compile time
+    __device__ __forceinline__ unsigned short pick(int d) const
+    {
+        const int k = d <= 13 ? d : 26 - d;
+        uint32_t v = w[0];
+#pragma unroll
+        for (int e = 1; e < 14; ++e) v = k == e ? w[e] : v;
+        return static_cast<unsigned short>(d <= 13 ? v : v >> 16);
+    }
+};
+
 // Arithmetic type used with each storage type.
 template <typename S> struct ArithOf { using type = float; };
 template <> struct ArithOf<double> { using type = double; };

@@ -408,8 +408,13 @@ __device__ __forceinline__ const S* xface_edge_ptr(const S* edge, const Domain& 
 // it shares the instruction cache with the inner rows' code, so it selects one
 // address per pull without branches and visits the readers face by face: the
 // 32x16x16 in-place FP16-SR step takes 13.6 us against 18.5 us with the
-// per-direction branches, the 288x272x280 one the same.  FP32 and FP64 keep
-// the branches: their steps of small domains are 9 % slower this way.
+// per-direction branches, the 288x272x280 one the same.  The results are held
+// across the two passes of stores as 16-bit patterns (Bits27), half the
+// registers of the values: held as FP32 they spilled up to twice as much in
+// the one-cell kernels (FP16-SR odd 216/328 bytes against 88/104) and slowed
+// the inner rows' code beside them (288x272x140 FP16 in place 300.3 against
+// 291.6 us, 33^3 FP16-SR 15.2 against 14.1 us).  FP32 and FP64 keep the
+// branches: their steps of small domains are 9 % slower this way.
 
 // Pull of layout A with the values that leave the domain from the edge buffer.
 template <typename S, typename R>
@@ -435,13 +440,13 @@ __device__ __forceinline__ void load_face_cell(const StepArgs<S, R>& a, const Ce
     }
 }
 
-// Visits the clamp readers of cell c: fn(d, f_d, y) for each direction d and
-// boundary cell y whose clamped pull of d reads c (for_each_clamp_reader).
+// Visits the clamp readers of cell c: fn(pattern of f_d, d, y) for each direction d
+// and boundary cell y whose clamped pull of d reads c (for_each_clamp_reader).
 // A cell on one face has readers on that face only, for the nine directions
 // that leave through it; the subsets of two or three axes, for cells on an
 // edge of the domain, go through a rolled loop.
-template <typename R, class F>
-__device__ __forceinline__ void visit_clamp_readers(const Domain& D, const CellCoord& c, const R* f, F&& fn)
+template <typename S, class F>
+__device__ __forceinline__ void visit_clamp_readers(const Domain& D, const CellCoord& c, const Bits27<S>& f, F&& fn)
 {
     const bool xl = c.x == 0, xh = c.x == D.nx - 1, yl = c.y == 0, yh = c.y == D.ny - 1, zl = c.z == 0,
                zh = c.z == D.nz - 1;
@@ -452,7 +457,7 @@ __device__ __forceinline__ void visit_clamp_readers(const Domain& D, const CellC
             const int cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
             if ((axis == 0 ? cx : axis == 1 ? cy : cz) != side) continue;
             const int yx = axis == 0 ? c.x : c.x + cx, yy = axis == 1 ? c.y : c.y + cy, yz = axis == 2 ? c.z : c.z + cz;
-            if (inside(D, yx, yy, yz)) fn(d, f[d], yx, yy, yz);
+            if (inside(D, yx, yy, yz)) fn(f.at(d), d, yx, yy, yz);
         }
     };
     face(xl, 0, 1);
@@ -470,14 +475,12 @@ __device__ __forceinline__ void visit_clamp_readers(const Domain& D, const CellC
         const int leave = ((cx == 1 && xl) || (cx == -1 && xh) ? 1 : 0) | ((cy == 1 && yl) || (cy == -1 && yh) ? 2 : 0) |
                           ((cz == 1 && zl) || (cz == -1 && zh) ? 4 : 0);
         if ((leave & (leave - 1)) == 0) continue;
-        R v = f[0];
-#pragma unroll
-        for (int e = 1; e < 27; ++e) v = d == e ? f[e] : v;
+        const unsigned short v = f.pick(d);
 #pragma unroll 1
         for (int m = leave; m > 2; m = (m - 1) & leave) {   // the subsets of two or three leaving axes
             if ((m & (m - 1)) == 0) continue;
             const int yx = (m & 1) ? c.x : c.x + cx, yy = (m & 2) ? c.y : c.y + cy, yz = (m & 4) ? c.z : c.z + cz;
-            if (inside(D, yx, yy, yz)) fn(d, v, yx, yy, yz);
+            if (inside(D, yx, yy, yz)) fn(v, d, yx, yy, yz);
         }
     }
 }
@@ -547,10 +550,13 @@ __device__ __forceinline__ void aa_odd_cell(const StepArgs<S, R>& a, const CellC
         }
     } else {
         if constexpr (Is16<S>::value) {
-            put27_raw_if<S>(f, hc, [&](int d) { return a.dst.p[d] + (c.i + nb_off(D, d)); },
-                            [&](int d) { return inside(D, c.x + cx_of(d), c.y + cy_of(d), c.z + cz_of(d)); });
-            visit_clamp_readers(D, c, f, [&](int d, R v, int yx, int yy, int yz) {
-                put_raw(a.dst.p[d] + (yx + D.nx * (yy + D.ny * yz)), v, hc, d);
+            const Bits27<S> b(f, hc);
+#pragma unroll
+            for (int d = 0; d < 27; ++d)
+                if (inside(D, c.x + cx_of(d), c.y + cy_of(d), c.z + cz_of(d)))
+                    st16(a.dst.p[d] + (c.i + nb_off(D, d)), b.at(d));
+            visit_clamp_readers(D, c, b, [&](unsigned short v, int d, int yx, int yy, int yz) {
+                st16(a.dst.p[d] + (yx + D.nx * (yy + D.ny * yz)), v);
             });
         } else {
             for_dirs([&](auto dd) {
@@ -584,6 +590,15 @@ __device__ __forceinline__ void aa_even_cell(const StepArgs<S, R>& a, const Cell
     }
     cell_update_for<S, true>(op, a.inv_tau, a.rho, a.vx, a.vy, a.vz, c.i, f);
     if (!(op & OP_STORE)) return;
+    if constexpr (ROWS == ROWS_OUTER && Is16<S>::value) {
+        const Bits27<S> b(f, hc);
+#pragma unroll
+        for (int d = 0; d < 27; ++d) st16(a.dst.p[26 - d] + c.i, b.at(d));
+        visit_clamp_readers(D, c, b, [&](unsigned short v, int d, int yx, int yy, int yz) {
+            st16(a.edge + edge_slot(D, a.el, yx, yy, yz, d), v);
+        });
+        return;
+    }
     put27_raw<S>(f, hc, [&](int d) { return a.dst.p[26 - d] + c.i; });
     if (ROWS == ROWS_INNER) {
         if (c.x != 0 && c.x != D.nx - 1) return;
@@ -598,18 +613,12 @@ __device__ __forceinline__ void aa_even_cell(const StepArgs<S, R>& a, const Cell
                         d);
         }
     } else {
-        if constexpr (Is16<S>::value) {
-            visit_clamp_readers(D, c, f, [&](int d, R v, int yx, int yy, int yz) {
-                put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), v, hc, d);
+        for_dirs([&](auto dd) {
+            constexpr int d = decltype(dd)::value;
+            for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
+                put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), f[d], hc, d);
             });
-        } else {
-            for_dirs([&](auto dd) {
-                constexpr int d = decltype(dd)::value;
-                for_each_clamp_reader<d>(D, c.x, c.y, c.z, [&](int yx, int yy, int yz) {
-                    put_raw(a.edge + edge_slot(D, a.el, yx, yy, yz, d), f[d], hc, d);
-                });
-            });
-        }
+        });
     }
 }
 
