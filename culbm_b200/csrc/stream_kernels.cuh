@@ -67,6 +67,7 @@ struct StepArgs {
     int ring_nz;   // LAYOUT_PULL_RING: planes in the ring buffer
     int ring_off;  // LAYOUT_PULL_RING: ring plane of domain plane z = 0
     uint32_t seed; // step_seed of the time step being written (stochastic rounding)
+    int overlap;   // in-place: the next step's blocks may start while this one's run (step_enter)
 };
 
 __device__ __forceinline__ int nb_off(const Domain& D, int d)
@@ -229,12 +230,13 @@ __device__ __forceinline__ void load_pulled(const StepArgs<S, R>& a, int x, int 
 // Programmatic dependent launch: consecutive steps are launched with
 // programmatic stream serialisation (launch_step), so the next step's blocks
 // may start while this grid's last blocks run.  Each step lets its dependents
-// start at once and waits for the previous grid (complete, its memory
-// visible) before touching memory; the wait is the hardware's own and always
-// ends.  Launched the ordinary way, both instructions do nothing.
-__device__ __forceinline__ void step_enter()
+// start at once (`overlap`; else each block as it ends) and waits for the
+// previous grid (complete, its memory visible) before touching memory; the
+// wait is the hardware's own and always ends.  Launched the ordinary way, both
+// instructions do nothing.
+__device__ __forceinline__ void step_enter(bool overlap = true)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (overlap) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -630,7 +632,7 @@ __device__ __forceinline__ void aa_even_cell(const StepArgs<S, R>& a, const Cell
 template <typename S, typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_aa_odd(const __grid_constant__ StepArgs<S, R> a)
 {
-    step_enter();
+    step_enter(a.overlap != 0);
     CellCoord c;
     const int kind = split_cell(a.dom, 0, c);
     if (kind == ROWS_OUTER)
@@ -642,7 +644,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_aa_odd(const __
 template <typename S, typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_aa_even(const __grid_constant__ StepArgs<S, R> a)
 {
-    step_enter();
+    step_enter(a.overlap != 0);
     CellCoord c;
     const int kind = split_cell(a.dom, 0, c);
     if (kind == ROWS_OUTER)
