@@ -8,19 +8,26 @@
 // (packed2.cuh): 453 instructions per cell.  The pulled values stay in their
 // stored form and are widened twice, once for the moments and once for the
 // relaxation, and each pair of directions is narrowed and stored as soon as
-// it is relaxed, so that the two cells fit 80 registers (six blocks of 128;
-// at 128 registers the pull runs a fifth slower, at 64 it spills).  All loads
-// are issued before the op bytes are looked at.  Threads take the pairs of a
-// plane (in place: of its inner rows) in memory order, so warps are full
-// whatever nx is.  Equilibrium cells (the row's ends of an inlet: a fifth of
-// the warps at nx = 288) run with the fluid cells in the packed code; walls
-// and other cells take the one-cell code after it.
+// it is relaxed, so that the two cells run at 80 registers (six blocks of 128;
+// at 128 registers the pull runs a fifth slower, at 64 it spills more).
+// Threads take the pairs of a plane (in place: of its inner rows) in memory
+// order, so warps are full whatever nx is.  Equilibrium cells (the row's ends
+// of an inlet: a fifth of the warps at nx = 288) run with the fluid cells in
+// the packed code.
 //
-// FP16-SR channel with spheres, 288x272x280: pull 585 -> 478 us per step
-// (45.9k MLUPS, 0.76 of the copy bandwidth), in place 666 -> 596 us; 512x512x256
-// 1744 -> 1428 us and 1948 -> 1729 us.  What bounds them now: latency (24 warps
-// per SM, 53 % issue, loads waited for first) and, in place, instruction
-// fetches besides (face rows and inner rows are two large bodies of code).
+// Each kernel comes in two codes.  The one for fluid issues all loads before
+// the op bytes are looked at, and leaves walls and other cells to the one-cell
+// code after it.  The one for mixed domains (mixed_domain, sim.cu) looks first
+// and leaves the loads of idle pairs out; walls run along in the packed code,
+// their stored values reversed, and a cell's half of a word is stored alone
+// where the other cell is not packed.  256x256x160 FP16-SR, pull and in place,
+// fluid code -> mixed code (one cell per thread): 60 % walls in blocks of 5^3
+// cells 373 -> 239 us (283) and 444 -> 298 (326), seven eighths idle 131 -> 64
+// (76) and 111 -> 71 (98).  One kernel with both codes runs fluid 7 % slower.
+//
+// FP16-SR channel with spheres, 288x272x280: pull 591 -> 476 us per step
+// (46.1k MLUPS, 0.76 of the copy bandwidth), in place 663 -> 590 us; 512x512x256
+// in place 1942 -> 1709 us.
 //
 // Odd nx keeps the one-cell kernels: without words the same code needs 108
 // 16-bit accesses per pair instead of 72, and the load/store units then bound
@@ -37,8 +44,10 @@ namespace culbm {
 
 constexpr int kCells2Threads = 128, kCells2Blocks = 6;
 
-// Division of 0 <= n < 2^31 by a divisor fixed on the host (rounded-up
-// reciprocal; n + umulhi(n, m) stays below 2^32).
+// Division of 0 <= n < 2^31 by a divisor fixed on the host, by Granlund and
+// Montgomery's multiplication with the rounded-up reciprocal ("Division by
+// invariant integers using multiplication", 1994); n + umulhi(n, m) stays
+// below 2^32.
 struct FastDiv {
     uint32_t m, s;
     __host__ void set(uint32_t d)
@@ -110,27 +119,37 @@ __device__ __forceinline__ CellCoord cell_in_pair(const Pair& c, int k)
     return {c.x + k, c.y, c.z, c.i + k, true};
 }
 
-// Cells of the packed code: plain fluid (LOAD, COLLIDE, STORE) and
-// equilibrium cells (EQU, STORE).
+// Cells of the packed code: plain fluid (LOAD, COLLIDE, STORE), equilibrium
+// cells (EQU, STORE) and, in the code for mixed domains, walls (LOAD,
+// bounce-back, STORE).
 __device__ __forceinline__ bool op_fluid(uint32_t op) { return (op & 0x1Fu) == (OP_LOAD | OP_COLLIDE | OP_STORE); }
 __device__ __forceinline__ bool op_equ(uint32_t op) { return (op & (0x1Fu ^ OP_LOAD)) == (OP_EQU | OP_STORE); }
+__device__ __forceinline__ bool op_wall(uint32_t op) { return (op & 0x1Fu) == (OP_LOAD | OP_BB | OP_STORE); }
 
 struct PairKind {
     bool e0, e1;    // cell 0, 1 is an equilibrium cell
+    bool b0, b1;    // cell 0, 1 is a wall (mixed domains)
     bool p0, p1;    // cell 0, 1 goes through the packed code
     bool equ;       // some lane of the warp has an equilibrium cell
+    bool wall;      // some lane of the warp has a wall (mixed domains)
     bool all;       // every cell of the warp's pairs goes through the packed code
 };
 
+// The votes are over whichever lanes arrive together: they choose between
+// codes with the same results.
+template <bool MIXED>
 __device__ __forceinline__ PairKind pair_kind(uint32_t ops)
 {
     PairKind k;
     k.e0 = op_equ(ops);
     k.e1 = op_equ(ops >> 8);
-    k.p0 = k.e0 || op_fluid(ops);
-    k.p1 = k.e1 || op_fluid(ops >> 8);
+    k.b0 = MIXED && op_wall(ops);
+    k.b1 = MIXED && op_wall(ops >> 8);
+    k.p0 = k.e0 || k.b0 || op_fluid(ops);
+    k.p1 = k.e1 || k.b1 || op_fluid(ops >> 8);
     const unsigned lanes = __activemask();
     k.equ = __any_sync(lanes, k.e0 || k.e1);
+    k.wall = MIXED && __any_sync(lanes, k.b0 || k.b1);
     k.all = __all_sync(lanes, k.p0 && k.p1);
     return k;
 }
@@ -150,7 +169,7 @@ __device__ __forceinline__ void prefetch_equ(const StepArgs<S, float>& a, const 
 // 26 - k in bits 16-31 (k = 13: both in bits 0-15).  An equilibrium cell runs
 // as a fluid cell with zero pulled values, its own rho and u, w = 1 and
 // 1 - w = -0: -0 * 0 + feq is feq to the sign of a zero.
-template <typename S, class F>
+template <typename S, bool MIXED, class F>
 __device__ __forceinline__ void relax_two(const StepArgs<S, float>& a, const PairKind& kind, int i, f32x2 z0,
                                           uint32_t* w, F&& emit)
 {
@@ -185,12 +204,19 @@ __device__ __forceinline__ void relax_two(const StepArgs<S, float>& a, const Pai
             put(t.om, -0.0f, -0.0f);
         },
         [&](int k, f32x2 fk, f32x2 fe) {
-            if (k < 13)
-                emit(k, Pack2<S>::cvt(lo2(fe), lo2(fk), IsSR<S>::value ? sr_word_pair(h0, k) : 0u),
-                     Pack2<S>::cvt(hi2(fe), hi2(fk), IsSR<S>::value ? sr_word_pair(h1, k) : 0u));
-            else
-                emit(13, static_cast<uint32_t>(enc16_raw<S>(lo2(fk), h0, 13)),
-                     static_cast<uint32_t>(enc16_raw<S>(hi2(fk), h1, 13)));
+            uint32_t v0, v1;
+            if (k < 13) {
+                v0 = Pack2<S>::cvt(lo2(fe), lo2(fk), IsSR<S>::value ? sr_word_pair(h0, k) : 0u);
+                v1 = Pack2<S>::cvt(hi2(fe), hi2(fk), IsSR<S>::value ? sr_word_pair(h1, k) : 0u);
+            } else {
+                v0 = enc16_raw<S>(lo2(fk), h0, 13);
+                v1 = enc16_raw<S>(hi2(fk), h1, 13);
+            }
+            if (MIXED && kind.wall) {   // a wall's stored values as they are, reversed
+                if (kind.b0) v0 = __byte_perm(w[26 - k], w[k], 0x5410);
+                if (kind.b1) v1 = __byte_perm(w[26 - k], w[k], 0x7632);
+            }
+            emit(k, v0, v1);
         });
 }
 
@@ -205,6 +231,9 @@ __device__ __forceinline__ void other_cells(bool done0, bool done1, F&& one)
 #pragma unroll 1
     for (int k = done0 ? 1 : 0, r = 0; r < rounds; ++r, ++k) one(k);
 }
+
+// A cell that does not store changes nothing.
+__device__ __forceinline__ bool op_keeps(uint32_t op) { return (op & OP_STORE) == 0; }
 
 // Direction d of an emitted pair: its two values as one word, or one cell's value.
 __device__ __forceinline__ uint32_t both_of(int d, uint32_t p, uint32_t q)
@@ -232,18 +261,68 @@ __device__ __forceinline__ void st_packed(const PairKind& k, S* p, int d, uint32
         st16(p + (k.p1 ? 1 : 0), one_of(d, k.p1 ? v1 : v0));
 }
 
+// Whether a cell of the pair loads.
+__device__ __forceinline__ bool pair_loads(uint32_t ops) { return (ops & (OP_LOAD | OP_LOAD << 8)) != 0; }
+
 // Op bytes of a pair (cell 0 in bits 0-7).
 __device__ __forceinline__ uint32_t ops_of(const uint8_t* ops, int i)
 {
     return *reinterpret_cast<const unsigned short*>(ops + i);
 }
 
-// One pull step src -> dst over the planes z0 + blockIdx.y.  An x-face cell
-// pulls the directions whose source lies outside from its own column: the
-// value the other cell of the pair pulls.  Its load past the row's side is
-// not used; it stays inside the 27 planes (cx = +1 has d >= 2, cx = -1 has
-// d <= 24).
-template <typename S>
+// The pull step src -> dst of a pair.  An x-face cell pulls the directions
+// whose source lies outside from its own column: the value the other cell of
+// the pair pulls.  Its load past the row's side is not used; it stays inside
+// the 27 planes (cx = +1 has d >= 2, cx = -1 has d <= 24).
+template <bool MIXED, typename S>
+__device__ __forceinline__ void pull_pair(const StepArgs<S, float>& a, const Pair& c, f32x2 nzero)
+{
+    const Domain& D = a.dom;
+    const uint32_t ops = ops_of(a.ops, c.i);
+    const int ym = c.y == 0 ? 0 : -D.nx, yp = c.y == D.ny - 1 ? 0 : D.nx;
+    const int zm = c.z == 0 ? 0 : -D.nxy, zp = c.z == D.nz - 1 ? 0 : D.nxy;
+    uint32_t w[27];   // not mixed: loaded before the op bytes are looked at
+    if (!MIXED || pair_loads(ops)) {
+#pragma unroll
+        for (int d = 0; d < 27; ++d) {
+            const int oy = cy_of(d) == 1 ? ym : cy_of(d) == -1 ? yp : 0;
+            const int oz = cz_of(d) == 1 ? zm : cz_of(d) == -1 ? zp : 0;
+            const S* p = a.src.p[d] + (c.i + oy + oz);
+            if (cx_of(d) == 0) {
+                w[d] = ld_word(p);
+            } else {
+                const uint32_t u = ld_half(p - cx_of(d)), v = ld_half(p + 1 - cx_of(d));
+                w[d] = cx_of(d) == 1 ? __byte_perm(c.lo ? v : u, v, 0x5410) : __byte_perm(u, c.hi ? u : v, 0x5410);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int d = 0; d < 27; ++d) w[d] = 0;
+    }
+    const PairKind kind = pair_kind<MIXED>(ops);
+    prefetch_equ(a, kind, c.i);
+    auto one = [&](int k) { pull_cell<S, float>(a, cell_in_pair(c, k)); };
+    if (MIXED) {
+        if (kind.p0 || kind.p1)
+            relax_two<S, MIXED>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
+                st_packed(kind, a.dst.p[k] + c.i, k, v0, v1);
+                if (k < 13) st_packed(kind, a.dst.p[26 - k] + c.i, 26 - k, v0, v1);
+            });
+        other_cells(kind.p0 || op_keeps(ops), kind.p1 || op_keeps(ops >> 8), one);
+    } else {
+        // the packed result of a cell outside the packed code is overwritten below; one without STORE keeps its slots
+        const bool packed = (kind.p0 || kind.p1) && (ops & (ops >> 8) & OP_STORE);
+        if (packed)
+            relax_two<S, MIXED>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
+                st_two(a.dst.p[k] + c.i, k, v0, v1);
+                if (k < 13) st_two(a.dst.p[26 - k] + c.i, 26 - k, v0, v1);
+            });
+        other_cells(kind.p0 && packed, kind.p1 && packed, one);
+    }
+}
+
+// One pull step over the planes z0 + blockIdx.y.
+template <typename S, bool MIXED>
 __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_pull_cells2(const __grid_constant__ StepArgs<S, float> a, FastDiv row, int z0, f32x2 nzero)
 {
@@ -252,32 +331,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     const uint32_t t = 2 * (blockIdx.x * kCells2Threads + threadIdx.x);   // cell 0 within the plane
     if (t >= static_cast<uint32_t>(D.nxy)) return;
     const Pair c = pair_at(D, row, static_cast<int>(t), z0 + static_cast<int>(blockIdx.y));
-    const uint32_t ops = ops_of(a.ops, c.i);
-    const int ym = c.y == 0 ? 0 : -D.nx, yp = c.y == D.ny - 1 ? 0 : D.nx;
-    const int zm = c.z == 0 ? 0 : -D.nxy, zp = c.z == D.nz - 1 ? 0 : D.nxy;
-    uint32_t w[27];   // loaded before the op bytes are looked at
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        const int oy = cy_of(d) == 1 ? ym : cy_of(d) == -1 ? yp : 0;
-        const int oz = cz_of(d) == 1 ? zm : cz_of(d) == -1 ? zp : 0;
-        const S* p = a.src.p[d] + (c.i + oy + oz);
-        if (cx_of(d) == 0) {
-            w[d] = ld_word(p);
-        } else {
-            const uint32_t u = ld_half(p - cx_of(d)), v = ld_half(p + 1 - cx_of(d));
-            w[d] = cx_of(d) == 1 ? __byte_perm(c.lo ? v : u, v, 0x5410) : __byte_perm(u, c.hi ? u : v, 0x5410);
-        }
-    }
-    const PairKind kind = pair_kind(ops);
-    prefetch_equ(a, kind, c.i);
-    // the packed result of a cell outside the packed code is overwritten below; one without STORE keeps its slots
-    const bool packed = (kind.p0 || kind.p1) && (ops & (ops >> 8) & OP_STORE);
-    if (packed)
-        relax_two<S>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
-            st_two(a.dst.p[k] + c.i, k, v0, v1);
-            if (k < 13) st_two(a.dst.p[26 - k] + c.i, 26 - k, v0, v1);
-        });
-    other_cells(kind.p0 && packed, kind.p1 && packed, [&](int k) { pull_cell<S, float>(a, cell_in_pair(c, k)); });
+    pull_pair<MIXED>(a, c, nzero);
 }
 
 // Launch of an in-place step over the planes of a SlabSplit: first `faces`
@@ -354,36 +408,32 @@ __device__ __forceinline__ S* xface_slot(const StepArgs<S, float>& a, int d, int
     return const_cast<S*>(xface_edge_ptr(a.edge, a.dom, a.el, cx_of(d) == 1 ? 0 : 1, d, y, z));
 }
 
-// In-place odd step (aa_odd_cell) of the inner rows' pairs.
-template <typename S>
-__global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
-    k_aa_odd_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
+// In-place odd step (aa_odd_cell) of a pair in the inner rows.
+template <bool MIXED, typename S>
+__device__ __forceinline__ void aa_odd_pair(const StepArgs<S, float>& a, const Pair& c, f32x2 nzero)
 {
     const Domain& D = a.dom;
-    step_enter();
-    if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
-        CellCoord c;
-        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_odd_cell<S, float, ROWS_OUTER>(a, c);
-        return;
-    }
-    Pair c;
-    if (!inner_pair(D, g, blockIdx.x - static_cast<uint32_t>(g.faces), c)) return;
     const uint32_t ops = ops_of(a.ops, c.i);
-    uint32_t w[27];   // loaded before the op bytes are looked at
+    uint32_t w[27];   // not mixed: loaded before the op bytes are looked at
+    if (!MIXED || pair_loads(ops)) {
 #pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        const S* p = a.src.p[26 - d] + (c.i - nb_off(D, d));
-        if (cx_of(d) == 0) {
-            w[d] = ld_word(p);
-        } else {
-            // the value of a face cell whose source lies outside comes from the edge buffer below
-            uint32_t u = 0, v = 0;
-            if (!(cx_of(d) == 1 && c.lo)) u = ld_half(p);
-            if (!(cx_of(d) == -1 && c.hi)) v = ld_half(p + 1);
-            w[d] = __byte_perm(u, v, 0x5410);
+        for (int d = 0; d < 27; ++d) {
+            const S* p = a.src.p[26 - d] + (c.i - nb_off(D, d));
+            if (cx_of(d) == 0) {
+                w[d] = ld_word(p);
+            } else {
+                // the value of a face cell whose source lies outside comes from the edge buffer below
+                uint32_t u = 0, v = 0;
+                if (!(cx_of(d) == 1 && c.lo)) u = ld_half(p);
+                if (!(cx_of(d) == -1 && c.hi)) v = ld_half(p + 1);
+                w[d] = __byte_perm(u, v, 0x5410);
+            }
         }
+    } else {
+#pragma unroll
+        for (int d = 0; d < 27; ++d) w[d] = 0;
     }
-    const PairKind kind = pair_kind(ops);
+    const PairKind kind = pair_kind<MIXED>(ops);
     const bool f0 = kind.p0, f1 = kind.p1;
     if (f0 || f1) {
         prefetch_equ(a, kind, c.i);
@@ -395,7 +445,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
 #pragma unroll
             for (int d = 0; d < 27; d += 3) w[d] = __byte_perm(w[d], ld_half(xface_slot(a, d, c.y, c.z)), 0x5410);
         }
-        relax_two<S>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
+        relax_two<S, MIXED>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
             auto out = [&](int d) {
                 S* p = a.dst.p[d] + (c.i + nb_off(D, d));
                 if (cx_of(d) == 0) {
@@ -414,32 +464,43 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
             if (k < 13) out(26 - k);
         });
     }
-    other_cells(f0, f1, [&](int k) { aa_odd_cell<S, float, ROWS_INNER_ONE>(a, cell_in_pair(c, k)); });
+    other_cells(f0 || (MIXED && op_keeps(ops)), f1 || (MIXED && op_keeps(ops >> 8)), [&](int k) { aa_odd_cell<S, float, ROWS_INNER_ONE>(a, cell_in_pair(c, k)); });
 }
 
-// In-place even step (aa_even_cell) of the inner rows' pairs.
-template <typename S>
+template <typename S, bool MIXED>
 __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
-    k_aa_even_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
+    k_aa_odd_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
 {
     const Domain& D = a.dom;
     step_enter();
     if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
         CellCoord c;
-        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_even_cell<S, float, ROWS_OUTER>(a, c);
+        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_odd_cell<S, float, ROWS_OUTER>(a, c);
         return;
     }
     Pair c;
     if (!inner_pair(D, g, blockIdx.x - static_cast<uint32_t>(g.faces), c)) return;
+    aa_odd_pair<MIXED>(a, c, nzero);
+}
+
+// In-place even step (aa_even_cell) of a pair in the inner rows.
+template <bool MIXED, typename S>
+__device__ __forceinline__ void aa_even_pair(const StepArgs<S, float>& a, const Pair& c, f32x2 nzero)
+{
     const uint32_t ops = ops_of(a.ops, c.i);
-    uint32_t w[27];   // loaded before the op bytes are looked at
+    uint32_t w[27];   // not mixed: loaded before the op bytes are looked at
+    if (!MIXED || pair_loads(ops)) {
 #pragma unroll
-    for (int d = 0; d < 27; ++d) w[d] = ld_word(a.src.p[d] + c.i);
-    const PairKind kind = pair_kind(ops);
+        for (int d = 0; d < 27; ++d) w[d] = ld_word(a.src.p[d] + c.i);
+    } else {
+#pragma unroll
+        for (int d = 0; d < 27; ++d) w[d] = 0;
+    }
+    const PairKind kind = pair_kind<MIXED>(ops);
     const bool f0 = kind.p0, f1 = kind.p1;
     if (f0 || f1) {
         prefetch_equ(a, kind, c.i);
-        relax_two<S>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
+        relax_two<S, MIXED>(a, kind, c.i, nzero, w, [&](int k, uint32_t v0, uint32_t v1) {
             st_packed(kind, a.dst.p[26 - k] + c.i, k, v0, v1);
             if (k < 13) st_packed(kind, a.dst.p[k] + c.i, 26 - k, v0, v1);
         });
@@ -452,7 +513,23 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
         if (c.lo && f0) file(2, 0);
         if (c.hi && f1) file(0, 1);
     }
-    other_cells(f0, f1, [&](int k) { aa_even_cell<S, float, ROWS_INNER>(a, cell_in_pair(c, k)); });
+    other_cells(f0 || (MIXED && op_keeps(ops)), f1 || (MIXED && op_keeps(ops >> 8)), [&](int k) { aa_even_cell<S, float, ROWS_INNER>(a, cell_in_pair(c, k)); });
+}
+
+template <typename S, bool MIXED>
+__global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
+    k_aa_even_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
+{
+    const Domain& D = a.dom;
+    step_enter();
+    if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
+        CellCoord c;
+        if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_even_cell<S, float, ROWS_OUTER>(a, c);
+        return;
+    }
+    Pair c;
+    if (!inner_pair(D, g, blockIdx.x - static_cast<uint32_t>(g.faces), c)) return;
+    aa_even_pair<MIXED>(a, c, nzero);
 }
 
 }  // namespace culbm

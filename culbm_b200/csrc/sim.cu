@@ -407,10 +407,40 @@ bool two_cells(const Domain& D)
     return Is16<S>::value && D.nx % 2 == 0;
 }
 
-// One pull step of the planes [za, zb) in the arguments' buffers; `follows`:
-// the launch before it on the stream is a step of the same call.
+// Whether the two-cell kernels run their code for mixed domains: where more
+// than one in eight of the row segments of 32 cells hold a cell that neither
+// collides nor takes an equilibrium (walls and idle cells).  Warps with such
+// cells cost the code for fluid, which loads first and takes walls cell by cell:
+// 256x256x160 FP16-SR pull with 60 % walls in blocks of 5^3 cells 373 us against
+// 239, seven eighths idle 131 against 64, half the cells idle one by one 424
+// against 289; fluid alone runs 6 to 10 % slower in the other code (288x272x280
+// 476 against 521), so the two meet at 15 to 20 % of such warps.  512 segments
+// of the caller's flags, spread over the domain, are looked at (all where there
+// are no more): 10 us of a load, and an estimate is enough for a speed.
+bool mixed_domain(const culbm_sim* s, const uint32_t* flag)
+{
+    const Domain& D = s->dom;
+    if (flag == nullptr || s->esize != 2 || D.nx % 2 != 0) return false;   // NULL: fluid everywhere
+    const uint64_t row = (static_cast<uint64_t>(D.nx) + 31) / 32, all = row * D.ny * D.nz;
+    const uint64_t looks = std::min<uint64_t>(all, 512);
+    uint64_t found = 0;
+    for (uint64_t k = 0; k < looks; ++k) {
+        // fractional parts of multiples of the golden ratio: even, and in step with no row or plane
+        const uint64_t seg = all == looks ? k : (k * 0x9E3779B97F4A7C15ull >> 32) * all >> 32;
+        const int x0 = static_cast<int>(seg % row) * 32;
+        const uint32_t* f = flag + seg / row * D.nx + x0;
+        bool other = false;
+        for (int x = 0; x < std::min(32, D.nx - x0); ++x) other = other || !(f[x] & (FLAG_COLLIDE | FLAG_EQU));
+        found += other;
+    }
+    return 8 * found > looks;
+}
+
+// One pull step of the planes [za, zb) in the arguments' buffers; `mixed`: of
+// a domain of that kind (mixed_domain); `follows`: the launch before it on the
+// stream is a step of the same call.
 template <typename S, typename R>
-culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t st, bool follows = false)
+culbm_status launch_pull(const StepArgs<S, R>& a, bool mixed, int za, int zb, cudaStream_t st, bool follows = false)
 {
     const Domain& D = a.dom;
     if constexpr (Is16<S>::value) {
@@ -419,7 +449,8 @@ culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t s
             row.set(static_cast<uint32_t>(D.nx));
             const long long per_block = 2ll * kCells2Threads;
             const dim3 g(static_cast<unsigned>((D.nxy + per_block - 1) / per_block), zb - za);
-            CULBM_CUDA(launch_step(follows, g, kCells2Threads, st, k_pull_cells2<S>, a, row, za, kNegZero2));
+            auto kern = mixed ? k_pull_cells2<S, true> : k_pull_cells2<S, false>;
+            CULBM_CUDA(launch_step(follows, g, kCells2Threads, st, kern, a, row, za, kNegZero2));
             return CULBM_OK;
         }
     }
@@ -430,14 +461,16 @@ culbm_status launch_pull(const StepArgs<S, R>& a, int za, int zb, cudaStream_t s
 
 // One in-place step of the planes [za, zb) (odd: layout A -> B).
 template <typename S, typename R>
-culbm_status launch_inplace(const StepArgs<S, R>& a, bool odd, int za, int zb, cudaStream_t st, bool follows = false)
+culbm_status launch_inplace(const StepArgs<S, R>& a, bool mixed, bool odd, int za, int zb, cudaStream_t st,
+                            bool follows = false)
 {
     const Domain& D = a.dom;
     if constexpr (Is16<S>::value) {
         if (two_cells<S>(D)) {
             long long blocks = 0;
             const Cells2Grid g = cells2_grid(D, za, zb, &blocks);
-            auto kern = odd ? k_aa_odd_cells2<S> : k_aa_even_cells2<S>;
+            auto kern = odd ? (mixed ? k_aa_odd_cells2<S, true> : k_aa_odd_cells2<S, false>)
+                            : (mixed ? k_aa_even_cells2<S, true> : k_aa_even_cells2<S, false>);
             CULBM_CUDA(launch_step(follows, static_cast<unsigned>(blocks), kCells2Threads, st, kern, a, g, kNegZero2));
             return CULBM_OK;
         }
@@ -542,12 +575,12 @@ culbm_status plain_steps(culbm_sim* s, uint32_t nsteps)
         if (!s->inplace) {
             auto a = make_args<S>(s, s->cur, 1 - s->cur);
             a.seed = seed;
-            CULBM_TRY((launch_pull<S, R>(a, 0, s->dom.nz, s->stream, k > 0)));
+            CULBM_TRY((launch_pull<S, R>(a, s->mixed, 0, s->dom.nz, s->stream, k > 0)));
             s->cur ^= 1;
         } else {
             auto a = make_args<S>(s, 0, 0);
             a.seed = seed;
-            CULBM_TRY((launch_inplace<S, R>(a, s->aa_phase == 0, 0, s->dom.nz, s->stream, k > 0)));
+            CULBM_TRY((launch_inplace<S, R>(a, s->mixed, s->aa_phase == 0, 0, s->dom.nz, s->stream, k > 0)));
             s->aa_phase ^= 1;
         }
         s->launches += 1;
@@ -644,6 +677,7 @@ culbm_status upload_state(culbm_sim* s, const uint32_t* flag, const float* const
 {
     const long long n = s->n;
     const dim3 g1(1184), b1(256);
+    s->mixed = mixed_domain(s, flag);
     if (flag != nullptr) {
         CULBM_CUDA(cudaMemcpyAsync(s->d_flag, flag, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
     } else {
@@ -810,11 +844,11 @@ culbm_status run_slab_steps(culbm_sim* s, int nslab, int nstream, int t0, int t1
             if (pull) {
                 auto a = make_args<S>(s, t & 1, 1 - (t & 1));
                 a.seed = step_seed(static_cast<uint32_t>(t));
-                CULBM_TRY((launch_pull<S, R>(a, za, zb, st)));
+                CULBM_TRY((launch_pull<S, R>(a, s->mixed, za, zb, st)));
             } else {
                 auto a = make_args<S>(s, 0, 0);
                 a.seed = step_seed(static_cast<uint32_t>(t));
-                CULBM_TRY((launch_inplace<S, R>(a, (t & 1) == 0, za, zb, st)));
+                CULBM_TRY((launch_inplace<S, R>(a, s->mixed, (t & 1) == 0, za, zb, st)));
             }
             s->launches += 1;
         }
@@ -853,6 +887,7 @@ culbm_status run_host_overlapped(culbm_sim* s, const uint32_t* flag, const float
     cudaStream_t h2d = s->copy_st[0], d2h = s->copy_st[1];
     const int T = static_cast<int>(nsteps);
 
+    s->mixed = mixed_domain(s, flag);
     // Everything follows the simulation's earlier work.
     CULBM_CUDA(cudaEventRecord(s->run_ev[0], s->stream));
     CULBM_CUDA(cudaStreamWaitEvent(h2d, s->run_ev[0], 0));

@@ -267,3 +267,85 @@ def test_warp_staged_wait_gives_up_and_reports(culbm):
         sim.synchronize()
         assert np.isfinite(sim.pulled_ddf()).all()
 
+
+
+def mixed_scene(dims, kind, inplace):
+    """A channel with, by kind: `few` walls, other and idle cells (less than one
+    row segment of 32 cells in eight), `porous` walls in blocks of three cells
+    in places on the x-faces, `idle` regions that neither load nor store with
+    equilibrium cells in them, or `each` kind of special cell one by one.  In
+    place, a cell without STORE keeps what its neighbours push into it, so
+    there walls stand between idle cells and fluid."""
+    sc = S.default_scene(*dims)
+    nx, ny, nz = dims
+    f = sc.flag
+    rng = np.random.default_rng(sum(dims) + len(kind))
+    f[:, :, 0] = S.EQUILIBRIUM
+    f[:, :, -1] = S.EQUILIBRIUM
+    sc.vx[:] = 0.02
+    idle = S.WALL if inplace else 0
+    if kind == "few":
+        for k, cell in enumerate((S.WALL, S.COLLIDE | S.STORE, idle, S.WALL, S.BOUNCE_BACK | S.STORE, S.FLUID)):
+            z, y = rng.integers(0, nz), rng.integers(0, ny)
+            f[z, y, 0 if k == 5 else rng.integers(0, nx)] = cell
+    elif kind == "porous":
+        blocks = rng.random((-(-nz // 3), -(-ny // 3), -(-nx // 3))) < 0.5
+        f[np.kron(blocks, np.ones((3, 3, 3)))[:nz, :ny, :nx] > 0] = S.WALL
+    elif kind == "idle":
+        f[:, ny // 3:, nx // 4:] = idle
+        f[:, ny // 3 + 1:, nx // 4 + 1:] = 0
+        f[:, ny // 3 + 1:, nx // 2] = S.EQUILIBRIUM
+    else:
+        for cell in (S.WALL, idle, S.COLLIDE | S.STORE, S.EQUILIBRIUM, S.LOAD | S.BOUNCE_BACK | S.COLLIDE | S.STORE):
+            f[rng.random(f.shape) < 0.15] = cell
+    return sc
+
+
+@pytest.mark.parametrize("storage", ["fp16", "bf16", "fp16sr", "bf16sr"])
+@pytest.mark.parametrize("kind", ["few", "porous", "idle", "each"])
+@pytest.mark.parametrize("dims", [(130, 12, 11), (66, 17, 9), (2, 11, 16)])
+def test_storage16_fluid_and_mixed_domains(culbm, orc, storage, kind, dims):
+    """The two codes of the two-cell kernels, for fluid and for domains with
+    many walls or idle cells: pull and in place, the whole domain and slab by
+    slab, against the oracle bit for bit (in place with idle cells: where cells
+    collide)."""
+    for sp in (0, 1):
+        sc = mixed_scene(dims, kind, sp == 1)
+        seen = np.ones(sc.n, bool) if sc.flag.all() or sp == 0 else (sc.flag.reshape(-1) & S.COLLIDE) != 0
+        for nsteps in (4, 5):
+            want = oracle_pulled16(orc, sc, storage, 0.7, nsteps).reshape(27, sc.n)
+            for slabs in (0, 3):
+                with culbm.Simulation(sc.shape, stream_policy=sp, inv_tau=0.7, storage=storage, run_slabs=slabs) as sim:
+                    if slabs:
+                        sim.run_host(nsteps, *sc.arrays())
+                    else:
+                        sim.load_state(*sc.arrays())
+                        sim.step(nsteps)
+                    got = sim.pulled_ddf().reshape(27, sc.n)
+                assert np.array_equal(bits(got[:, seen]), bits(want[:, seen])), (nsteps, sp, slabs)
+
+
+@pytest.mark.parametrize("storage", ["fp16", "bf16", "fp16sr", "bf16sr"])
+def test_storage16_walls_hand_on_every_pattern(culbm, orc, storage):
+    """Walls reverse what they pulled, every finite 16-bit pattern of it, zeros
+    of both signs and subnormals among them."""
+    sc = S.default_scene(64, 6, 7)
+    sc.flag[:] = S.WALL
+    n = 27 * sc.n
+    pattern = (np.arange(n, dtype=np.uint32) % 65536).astype(np.uint16)
+    pattern[(pattern & 0x7FFF) >= (0x7F80 if storage.startswith("bf") else 0x7C00)] = 0
+    if storage.startswith("bf"):
+        state = (pattern.astype(np.uint32) << 16).view(np.float32)
+    else:
+        state = pattern.view(np.float16).astype(np.float32) * np.float32(2.0 ** -15)
+    f, r, ux, uy, uz = sc.arrays()
+    o = orc.Scene(64, 6, 7, f, r, ux, uy, uz)
+    for nsteps in (1, 2):
+        want = orc.pulled(o, orc.run_s16(o, storage, 0.7, nsteps, state=state))
+        for sp in (0, 1):
+            with culbm.Simulation(sc.shape, stream_policy=sp, inv_tau=0.7, storage=storage) as sim:
+                sim.load_state(f, r, ux, uy, uz)
+                sim.set_ddf(state)
+                sim.step(nsteps)
+                got = sim.pulled_ddf()
+            assert np.array_equal(bits(got), bits(want)), (nsteps, sp)
