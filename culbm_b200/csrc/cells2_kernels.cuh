@@ -317,6 +317,8 @@ __device__ __forceinline__ void pull_pair(const StepArgs<S, float>& a, const Pai
                 st_two(a.dst.p[k] + c.i, k, v0, v1);
                 if (k < 13) st_two(a.dst.p[26 - k] + c.i, 26 - k, v0, v1);
             });
+        // its halves are stored after the words, as another type: nothing may move between
+        asm volatile("" ::: "memory");
         other_cells(kind.p0 && packed, kind.p1 && packed, one);
     }
 }
