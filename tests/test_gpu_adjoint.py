@@ -269,3 +269,29 @@ def test_equ_cells_change_between_gradients(storage):
             assert not got[3][:, (fl & S.EQU) == 0].any()
         info = kept.info()
         assert info["forward_ms"] > 0 and info["recompute_ms"] > 0 and info["adjoint_ms"] > 0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16", "fp64"])
+def test_idle_cells_beside_the_channel(storage):
+    """Cells that neither load nor store beyond a channel's wall change nothing
+    in it (the forward step has a code for domains with many of them): the
+    gradients of the channel alone, bit for bit."""
+    nx, ny, nz = 34, 9, 7
+    sc, f, r, ux, uy, uz, soft = case(nx, ny, nz, bumps=3)
+    out = []
+    for rows in (ny, 2 * ny):
+        def wide(a, fill):
+            b = np.full((nz, rows, nx), fill, a.dtype)
+            b[:, :ny] = a.reshape(nz, ny, nx)
+            return b.reshape(-1)
+
+        with AdjointProblem((nx, rows, nz), window=(6, 10), inv_tau=0.7, checkpoint_every=4, storage=storage,
+                            precision="fp64" if storage == "fp64" else "fp32") as p:
+            p.set_state(wide(f, 0), wide(r, 1), wide(ux, 0), wide(uy, 0), wide(uz, 0), wide(soft, 0))
+            J, g_tau, g_soft, g_mac = p.gradient()
+            assert p.forward() == J
+        out.append((J, g_tau, g_soft.reshape(nz, rows, nx)[:, :ny], g_mac.reshape(4, nz, rows, nx)[:, :, :ny]))
+    (J, g_tau, g_soft, g_mac), (Ji, g_taui, g_softi, g_maci) = out
+    # the plane and block sums (FP64) run in another order
+    assert abs(J - Ji) <= 1e-10 * abs(J) and abs(g_tau - g_taui) <= 1e-10 * abs(g_tau)
+    assert np.array_equal(g_soft, g_softi) and np.array_equal(g_mac, g_maci)
