@@ -132,7 +132,11 @@ def test_run_host_slab_counts(culbm, run_slabs, nsteps):
 
 def test_run_host_sequential_configurations(culbm):
     """The tile engine and the staged 16-bit kernels run the four calls in order."""
-    for dims, kw in (((37, 29, 23), dict(stream_policy=1, opt_policy=3, inner_loop=3, tile=(16, 12, 10))),
+    tiles = dict(opt_policy=3, inner_loop=3, tile=(16, 12, 10))
+    for dims, kw in (((37, 29, 23), dict(stream_policy=1, use_ring=True, **tiles)),
+                     ((37, 29, 23), dict(stream_policy=1, persist_l2=True, **tiles)),
+                     ((37, 29, 23), dict(stream_policy=0, persist_l2=True, **tiles)),
+                     ((37, 29, 23), dict(stream_policy=1, **tiles)),   # plain pull steps: overlapped
                      ((32, 12, 20), dict(stream_policy=0, storage="fp16sr", kernel_variant=1))):
         arrs = scene(dims).arrays()
         want = sequential(culbm, dims, arrs, 6, **kw)

@@ -22,18 +22,27 @@ def oracle_pulled16(orc, scene, storage, inv_tau, nsteps):
 
 
 @pytest.mark.parametrize("storage", ["fp16", "bf16", "fp16sr", "bf16sr"])
-@pytest.mark.parametrize("policy", [(0, 0), (1, 0), (1, 3), (0, 3)])
-def test_storage16_matches_oracle(culbm, orc, storage, policy):
+@pytest.mark.parametrize("policy,engine", [((0, 0), ""), ((1, 0), ""), ((1, 3), ""), ((0, 3), ""), ((1, 3), "persist_l2"),
+                                           ((0, 3), "persist_l2"), ((1, 3), "use_ring"), ((0, 2), "persist_l2")])
+def test_storage16_matches_oracle(culbm, orc, storage, policy, engine):
+    """Plain policies, blocked ones as plain pull steps and on the tile engine
+    (persisting-L2 window, ring buffer; optPolicy 2 with a tile that no cluster
+    holds), which shows in the launch count."""
     sc = S.reference_channel_cube(34, 22, 18, 0.05)
     sc.flag[0, :, :] = S.FLUID          # one fluid face: exercises the clamped edge too
     nsteps = 11
     want = oracle_pulled16(orc, sc, storage, 0.55, nsteps)
     sp, op = policy
     kw = dict(tile=(18, 14, 12), inner_loop=3) if op else {}
+    if op == 2:
+        kw["tile"] = (34, 22, 12)
+    if engine:
+        kw[engine] = True
     with culbm.Simulation(sc.shape, stream_policy=sp, opt_policy=op, inv_tau=0.55, storage=storage, **kw) as sim:
         sim.load_state(*sc.arrays())
         sim.step(nsteps)
         got = sim.pulled_ddf()
+        assert (sim.info()["launches_per_step"] > 1.0) == bool(engine)
     assert np.array_equal(bits(got), bits(want)), (storage, policy)
 
 
