@@ -682,13 +682,13 @@ struct culbm_adj {
     void* d_nu = nullptr;       // 2 x 27 N of the arithmetic type
     double* d_gsoft = nullptr;
     double* d_gtau = nullptr;
-    double* d_gmac = nullptr;   // 4 n_equ
+    double* d_gmac = nullptr;   // 4 N, of which 4 n_equ are used
     double* d_psum = nullptr;   // 2 per time step of the window
     double* d_rho_plane = nullptr;  // window x 2 planes x ny*nz
     long long n_tau_blocks = 0;     // warps of one adjoint-step launch (one FP64 slot each)
     long long tau_capacity = 0;
     int* d_equ = nullptr;           // EQU cells, increasing
-    int n_equ = 0, equ_capacity = 0, gmac_capacity = 0;
+    int n_equ = 0, equ_capacity = 0;
     int n_in = 0, n_out = 0;
     bool idle = false;              // more than one cell in sixteen does not load
     uint64_t device_bytes = 0;
@@ -1232,6 +1232,8 @@ culbm_status culbm_adj_create(const culbm_adj_config* cfg, culbm_adj** out)
         CULBM_TRY(adj_alloc(a, &a->d_nu, 2ull * 27 * n * a->rsize, "adjoint populations"));
         CULBM_TRY(adj_alloc(a, &p, n * sizeof(double), "soft gradient"));
         a->d_gsoft = static_cast<double*>(p);
+        CULBM_TRY(adj_alloc(a, &p, 4 * n * sizeof(double), "EQU input gradients"));
+        a->d_gmac = static_cast<double*>(p);
         const long long nt = c.window[1] - c.window[0] + 1;
         CULBM_TRY(adj_alloc(a, &p, 2ull * nt * sizeof(double), "objective sums"));
         a->d_psum = static_cast<double*>(p);
@@ -1304,17 +1306,11 @@ culbm_status culbm_adj_set_state(culbm_adj* a, const uint32_t* flag, const float
         CULBM_CUDA(cudaFree(a->d_equ));
         a->d_equ = nullptr;
         a->device_bytes -= a->equ_capacity * sizeof(int);
-        CULBM_CUDA(cudaFree(a->d_gmac));
-        a->d_gmac = nullptr;
-        a->device_bytes -= a->gmac_capacity * 4 * sizeof(double);
-        a->equ_capacity = a->gmac_capacity = 0;
+        a->equ_capacity = 0;
         void* p = nullptr;
         CULBM_TRY(adj_alloc(a, &p, n_equ * sizeof(int), "EQU cell list"));
         a->d_equ = static_cast<int*>(p);
         a->equ_capacity = n_equ;
-        CULBM_TRY(adj_alloc(a, &p, 4ull * n_equ * sizeof(double), "EQU input gradients"));
-        a->d_gmac = static_cast<double*>(p);
-        a->gmac_capacity = n_equ;
     }
     {
         const dim3 gr = adj::adj_grid(a->dom, n_equ);

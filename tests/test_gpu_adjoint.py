@@ -295,3 +295,51 @@ def test_idle_cells_beside_the_channel(storage):
     # the plane and block sums (FP64) run in another order
     assert abs(J - Ji) <= 1e-10 * abs(J) and abs(g_tau - g_taui) <= 1e-10 * abs(g_tau)
     assert np.array_equal(g_soft, g_softi) and np.array_equal(g_mac, g_maci)
+
+
+def _fail_at(gate):
+    """The next CUDA call but `gate` fails, with an injected error code."""
+    from culbm_b200 import _capi
+    _capi.lib().culbm_debug_inject_cuda_error(gate, 2)   # cudaErrorMemoryAllocation
+
+
+def _no_failure():
+    from culbm_b200 import _capi
+    _capi.lib().culbm_debug_inject_cuda_error(0, 0)
+
+
+def test_set_state_after_a_failure():
+    """culbm_adj_set_state with more EQU cells than before, failing at each of
+    its CUDA calls in turn: repeated, it works, and the gradient and the device
+    memory are a fresh handle's."""
+    from culbm_b200._capi import CulbmError
+    dims = (34, 9, 7)
+    sc, f, r, ux, uy, uz, soft = case(*dims, bumps=2)
+    few = f.copy()
+    few[(f & S.EQU) != 0] = S.FLUID
+
+    def problem():
+        return AdjointProblem(dims, window=(6, 10), inv_tau=0.7, checkpoint_every=4)
+
+    with problem() as fresh:
+        fresh.set_state(few, r, ux, uy, uz, soft)
+        fresh.set_state(f, r, ux, uy, uz, soft)
+        want, size = fresh.gradient(), fresh.info()["device_bytes"]
+    failures = 0
+    for gate in range(64):
+        with problem() as p:
+            p.set_state(few, r, ux, uy, uz, soft)
+            _fail_at(gate)
+            try:
+                p.set_state(f, r, ux, uy, uz, soft)
+            except CulbmError:
+                failures += 1
+            else:
+                break
+            finally:
+                _no_failure()
+            p.set_state(f, r, ux, uy, uz, soft)
+            for a, b in zip(p.gradient(), want):
+                assert np.array_equal(np.asarray(a), np.asarray(b)), gate
+            assert p.info()["device_bytes"] == size, gate
+    assert 8 < failures < 64
