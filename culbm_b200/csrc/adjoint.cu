@@ -30,6 +30,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -1104,6 +1105,39 @@ bool choose_plan(int T, long long max_states, CkptPlan& out)
     return have && best.states() <= max_states;
 }
 
+culbm_status gradient(culbm_adj* a, double* J, double* dJ_dinv_tau, double* dJ_dsoft, double* dJ_dmac)
+{
+    CULBM_CUDA(cudaSetDevice(a->dev));
+    const size_t n = static_cast<size_t>(a->n), m = static_cast<size_t>(a->n_equ);
+    std::vector<double> tau(static_cast<size_t>(a->n_tau_blocks)), mac(4 * m);
+    CULBM_TRY(adj_with_storage(a, [&](auto tag) { return run_gradient<typename decltype(tag)::type>(a); }));
+    // dJ/d(rho, u) is zero but at the EQU cells: only their values leave the
+    // device, and the zeros are written here while it computes (dJ/ds too,
+    // so that its copy meets mapped pages).  192x136x140: 28 -> 3 ms of the
+    // call spent on its outputs and on waits between segments.  Not before the
+    // device has all of the work: until then a failure leaves the outputs as
+    // they were.
+    ZeroFill zero;
+    zero.start(dJ_dsoft, n, dJ_dmac, 4 * n);
+    CULBM_TRY(read_marks(a));
+    double j = 0;
+    CULBM_TRY(objective(a, &j));
+    zero.wait();
+    CULBM_CUDA(cudaMemcpy(tau.data(), a->d_gtau, tau.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    if (m) CULBM_CUDA(cudaMemcpy(mac.data(), a->d_gmac, mac.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    if (dJ_dsoft) CULBM_CUDA(cudaMemcpy(dJ_dsoft, a->d_gsoft, n * sizeof(double), cudaMemcpyDeviceToHost));
+    if (dJ_dmac)
+        for (size_t k = 0; k < 4; ++k)
+            for (size_t q = 0; q < m; ++q) dJ_dmac[k * n + a->h_equ[q]] = mac[k * m + q];
+    if (dJ_dinv_tau) {
+        double s = 0;
+        for (double v : tau) s += v;
+        *dJ_dinv_tau = s;
+    }
+    if (J) *J = j;
+    return CULBM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1329,10 +1363,10 @@ culbm_status culbm_adj_set_state(culbm_adj* a, const uint32_t* flag, const float
         }
         a->n_tau_blocks = slots;
     }
-    a->n_equ = n_equ;
-    a->h_equ = equ;
     if (n_equ)
         CULBM_CUDA(cudaMemcpyAsync(a->d_equ, equ.data(), n_equ * sizeof(int), cudaMemcpyHostToDevice, a->stream));
+    a->h_equ.swap(equ);
+    a->n_equ = n_equ;
     CULBM_CUDA(cudaMemcpyAsync(a->d_ops, ops.data(), n, cudaMemcpyHostToDevice, a->stream));
     const float* mac[4] = {rho, vx, vy, vz};
     const float dflt[4] = {1.0f, 0.0f, 0.0f, 0.0f};
@@ -1382,36 +1416,11 @@ culbm_status culbm_adj_forward(culbm_adj* a, double* J)
 culbm_status culbm_adj_gradient(culbm_adj* a, double* J, double* dJ_dinv_tau, double* dJ_dsoft, double* dJ_dmac)
 {
     if (!a) return fail(CULBM_ERR_INVALID_ARGUMENT, "adjoint handle is NULL");
-    CULBM_CUDA(cudaSetDevice(a->dev));
-    const size_t n = static_cast<size_t>(a->n);
-    // dJ/d(rho, u) is zero but at the EQU cells: only their values leave the
-    // device, and the zeros are written here while it computes (dJ/ds too,
-    // so that its copy meets mapped pages).  192x136x140: 28 -> 3 ms of the
-    // call spent on its outputs and on waits between segments.
-    ZeroFill zero;
-    zero.start(dJ_dsoft, n, dJ_dmac, 4 * n);
-    CULBM_TRY(adj_with_storage(a, [&](auto tag) { return run_gradient<typename decltype(tag)::type>(a); }));
-    CULBM_TRY(read_marks(a));
-    double j = 0;
-    CULBM_TRY(objective(a, &j));
-    if (J) *J = j;
-    zero.wait();
-    if (dJ_dinv_tau) {
-        std::vector<double> g(static_cast<size_t>(a->n_tau_blocks));
-        CULBM_CUDA(cudaMemcpy(g.data(), a->d_gtau, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        double s = 0;
-        for (double v : g) s += v;
-        *dJ_dinv_tau = s;
+    try {
+        return gradient(a, J, dJ_dinv_tau, dJ_dsoft, dJ_dmac);
+    } catch (const std::bad_alloc&) {
+        return fail(CULBM_ERR_OUT_OF_MEMORY, "host memory for the gradient");
     }
-    if (dJ_dsoft) CULBM_CUDA(cudaMemcpy(dJ_dsoft, a->d_gsoft, n * sizeof(double), cudaMemcpyDeviceToHost));
-    if (dJ_dmac && a->n_equ) {
-        const size_t m = static_cast<size_t>(a->n_equ);
-        std::vector<double> g(4 * m);
-        CULBM_CUDA(cudaMemcpy(g.data(), a->d_gmac, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        for (size_t k = 0; k < 4; ++k)
-            for (size_t q = 0; q < m; ++q) dJ_dmac[k * n + a->h_equ[q]] = g[k * m + q];
-    }
-    return CULBM_OK;
 }
 
 culbm_status culbm_adj_get_info(culbm_adj* a, culbm_adj_info* info)

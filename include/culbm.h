@@ -447,6 +447,9 @@ culbm_status culbm_adj_forward(culbm_adj* adj, double* J);
  * Forward run, then the adjoint sweep.  Outputs (host, any may be NULL):
  * J; dJ/d invTau; dJ/ds per cell (N doubles, 0 where no COLLIDE); dJ/d of the
  * EQU inputs rho, vx, vy, vz per cell (4*N doubles, field-major, 0 where no EQU).
+ * They are written only after the device has taken all of the work: an error
+ * before that leaves them as they were, and one of the device itself after it
+ * leaves them undefined.
  */
 culbm_status culbm_adj_gradient(culbm_adj* adj, double* J, double* dJ_dinv_tau, double* dJ_dsoft,
                                 double* dJ_dmac);

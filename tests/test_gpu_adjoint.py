@@ -343,3 +343,41 @@ def test_set_state_after_a_failure():
                 assert np.array_equal(np.asarray(a), np.asarray(b)), gate
             assert p.info()["device_bytes"] == size, gate
     assert 8 < failures < 64
+
+
+def test_gradient_outputs_after_a_failure():
+    """culbm_adj_gradient failing at CUDA calls up to the submission of its last
+    launch leaves every output as it was; then it works as before."""
+    import ctypes as C
+
+    from culbm_b200 import _capi
+    dims = (34, 9, 7)
+    sc, f, r, ux, uy, uz, soft = case(*dims, bumps=2)
+    n = f.size
+    with AdjointProblem(dims, window=(20, 30), inv_tau=0.7, checkpoint_every=8) as p:
+        p.set_state(f, r, ux, uy, uz, soft)
+        want = p.gradient()
+
+        def failing(gate):
+            """Whether the call fails, and its outputs."""
+            out = [np.full(k, 3.25) for k in (1, 1, n, 4 * n)]
+            _fail_at(gate)
+            try:
+                status = _capi.lib().culbm_adj_gradient(p._h, *[a.ctypes.data_as(C.POINTER(C.c_double)) for a in out])
+            finally:
+                _no_failure()
+            return status != 0, out
+
+        lo, hi = 0, 1024                 # calls of one gradient
+        assert not failing(hi)[0]
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            lo, hi = (mid, hi) if failing(mid)[0] else (lo, mid)
+        # behind the last launch: the wait, the times of 11 marks, the objective, three copies
+        last = hi - 32
+        assert last > 50
+        for gate in [*range(8), *range(8, last, 7), last - 1]:
+            failed, out = failing(gate)
+            assert failed and all((a == 3.25).all() for a in out), gate
+        for a, b in zip(p.gradient(), want):
+            assert np.array_equal(np.asarray(a), np.asarray(b))
