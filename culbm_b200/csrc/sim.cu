@@ -407,16 +407,20 @@ bool two_cells(const Domain& D)
     return Is16<S>::value && D.nx % 2 == 0;
 }
 
-// Whether the two-cell kernels run their code for mixed domains: where more
-// than one in eight of the row segments of 32 cells hold a cell that neither
-// collides nor takes an equilibrium (walls and idle cells).  Warps with such
-// cells cost the code for fluid, which loads first and takes walls cell by cell:
-// 256x256x160 FP16-SR pull with 60 % walls in blocks of 5^3 cells 373 us against
-// 239, seven eighths idle 131 against 64, half the cells idle one by one 424
-// against 289; fluid alone runs 6 to 10 % slower in the other code (288x272x280
-// 476 against 521), so the two meet at 15 to 20 % of such warps.  512 segments
-// of the caller's flags, spread over the domain, are looked at (all where there
-// are no more): 10 us of a load, and an estimate is enough for a speed.
+// Whether the two-cell kernels run their code for mixed domains: by the share
+// of row segments of 32 cells that cost the code for fluid, which loads first
+// and takes walls cell by cell.  Pull: segments with a cell that neither
+// collides nor takes an equilibrium (a wall or an idle cell), more than one in
+// six.  In place, where idle cells among fluid and whole rows of walls cost the
+// fluid code little: segments with walls beside such cells, or with no cell
+// that loads or takes an equilibrium, more than one in five.
+// 256x256x160, fluid code against mixed code: 60 % walls in blocks of 5^3 cells in
+// 10, 15, 20 and 30 % of the planes FP16-SR 245/247, 252/246, 259/246 and 273/245 us
+// pull, 303/307, 311/307, 318/306 and 334/305 in place (FP16: 247/237 and
+// 293/287 at 10 %); idle planes 20 % 212/207 and 249/257, 30 % 201/187 and
+// 229/231; planes of walls 30 % 245/242 and 286/302.
+// 512 segments of the caller's flags, spread over the domain, are looked at (all
+// where there are no more): 10 us of a load, and an estimate is enough for a speed.
 bool mixed_domain(const culbm_sim* s, const uint32_t* flag)
 {
     const Domain& D = s->dom;
@@ -429,11 +433,17 @@ bool mixed_domain(const culbm_sim* s, const uint32_t* flag)
         const uint64_t seg = all == looks ? k : (k * 0x9E3779B97F4A7C15ull >> 32) * all >> 32;
         const int x0 = static_cast<int>(seg % row) * 32;
         const uint32_t* f = flag + seg / row * D.nx + x0;
-        bool other = false;
-        for (int x = 0; x < std::min(32, D.nx - x0); ++x) other = other || !(f[x] & (FLAG_COLLIDE | FLAG_EQU));
-        found += other;
+        bool flow = false, wall = false, other = false, idle = true;
+        for (int x = 0; x < std::min(32, D.nx - x0); ++x) {
+            const bool moves = (f[x] & (FLAG_COLLIDE | FLAG_EQU)) != 0;
+            flow = flow || moves;
+            other = other || !moves;
+            wall = wall || (!moves && (f[x] & FLAG_STORE));
+            idle = idle && !(f[x] & (FLAG_LOAD | FLAG_EQU));
+        }
+        found += s->inplace ? (wall && flow) || idle : other;
     }
-    return 8 * found > looks;
+    return (s->inplace ? 5 : 6) * found > looks;
 }
 
 // One pull step of the planes [za, zb) in the arguments' buffers; `mixed`: of
