@@ -61,6 +61,7 @@ struct Args {
     int plane_in, plane_out;
     R obj_in, obj_out;   // dJ/df_d of one in/out plane cell at this time (0 outside the window)
     uint32_t seed;
+    int overlap;         // the next step's blocks may start while this one's run (step_enter)
     double* rho_plane;   // forward: rho of the two measurement planes of the pulled state, this step
                          // (null outside the objective window); [2][ny*nz]
     double* g_tau_block; // adjoint: one FP64 accumulator per warp
@@ -134,7 +135,7 @@ template <typename S, typename R, bool IDLE>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) k_soft_step(const __grid_constant__ Args<S, R> a)
 {
     const CellCoord c = cell_of_thread(a.dom);
-    step_enter();
+    step_enter(a.overlap != 0);
     if (!c.valid) return;
     constexpr int E = ScaleExp<S>::value;
     const uint8_t op = a.ops[c.i];
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
     k_adj_step(const __grid_constant__ Args<S, R> a, AdjLayout L)
 {
     double gtau_local = 0.0;
-    step_enter();
+    step_enter(a.overlap != 0);
     if (static_cast<int>(blockIdx.z) < L.equ_z) {
         const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
         const int k = blk * 256 + threadIdx.x + 32 * threadIdx.y;
@@ -803,6 +804,9 @@ culbm_status forward_run(culbm_adj* a, int t_begin, int t_end, S* src, SlotOf sl
     const long long plane = 2ll * a->dom.ny * a->dom.nz;
     S* cur = src;
     auto kern = a->idle ? adj::k_soft_step<S, R, true> : adj::k_soft_step<S, R, false>;
+    bool overlap = true;
+    CULBM_CUDA(steps_overlap(a->dev, kern, 256, 1ll * grid.x * grid.y * grid.z, &overlap));
+    g.overlap = overlap;
     for (int t = t_begin; t < t_end; ++t) {
         S* dst = slot_of(t + 1);
         set_pops<S, R>(g.src, cur, a->n);
@@ -953,6 +957,9 @@ culbm_status adjoint_segment(culbm_adj* a, int tb, int te, S* start, adj::Args<S
     auto slot_of = [&](int t) -> S* { return state_ptr<S>(a, SEG, t - tb - 1); };
     if (!states_present) CULBM_TRY(forward_run<S>(a, tb, te - 1, start, slot_of, false));
     CULBM_TRY(mark(a, PHASE_RECOMPUTE));
+    bool overlap = true;
+    CULBM_CUDA(steps_overlap(a->dev, adj::k_adj_step<S, R>, 256, 1ll * gr.x * gr.y * gr.z, &overlap));
+    g.overlap = overlap;
     for (int t = te - 1; t >= tb; --t) {
         S* st = (t == tb) ? start : state_ptr<S>(a, SEG, t - tb - 1);
         set_pops<S, R>(g.src, st, a->n);

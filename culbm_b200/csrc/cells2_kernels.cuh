@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_pull_cells2(const __grid_constant__ StepArgs<S, float> a, FastDiv row, int z0, f32x2 nzero)
 {
     const Domain& D = a.dom;
-    step_enter();
+    step_enter(a.overlap != 0);
     const uint32_t t = 2 * (blockIdx.x * kCells2Threads + threadIdx.x);   // cell 0 within the plane
     if (t >= static_cast<uint32_t>(D.nxy)) return;
     const Pair c = pair_at(D, row, static_cast<int>(t), z0 + static_cast<int>(blockIdx.y));
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_aa_odd_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
 {
     const Domain& D = a.dom;
-    step_enter();
+    step_enter(a.overlap != 0);
     if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
         CellCoord c;
         if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_odd_cell<S, float, ROWS_OUTER>(a, c);
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kCells2Threads, kCells2Blocks)
     k_aa_even_cells2(const __grid_constant__ StepArgs<S, float> a, const __grid_constant__ Cells2Grid g, f32x2 nzero)
 {
     const Domain& D = a.dom;
-    step_enter();
+    step_enter(a.overlap != 0);
     if (blockIdx.x < static_cast<uint32_t>(g.faces)) {
         CellCoord c;
         if (face_cell(D, g, blockIdx.x * kCells2Threads + threadIdx.x, c)) aa_even_cell<S, float, ROWS_OUTER>(a, c);

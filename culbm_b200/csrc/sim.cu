@@ -80,7 +80,7 @@ StepArgs<S, typename ArithOf<S>::type> make_args(const culbm_sim* s, int src, in
     a.edge = static_cast<S*>(s->d_edge);
     a.el = s->el;
     a.seed = step_seed(static_cast<uint32_t>(s->step));
-    a.overlap = s->inplace_overlap;
+    a.overlap = s->overlap;
     return a;
 }
 
@@ -498,26 +498,29 @@ culbm_status launch_inplace(const StepArgs<S, R>& a, bool mixed, bool odd, int z
     return CULBM_OK;
 }
 
-// Whether the blocks of an in-place step (one cell per thread) start before
-// the step ahead of them ends: not when nearly the whole step is resident at
-// once.  The next step's blocks then take their places while this one's run,
-// wherever there is room, and crowd some SMs; a short step waits for its
-// fullest SM.  Started as blocks end: 12^3 FP32 8.8 us against 11.7 (launched
-// the ordinary way 11.3), 96x24x24 10.2 against 12.5 (12.0), 128x32x32 (1.05
-// times the resident blocks) 11.0 against 12.1, 25^3 FP16-SR 9.9 against 11.8.
-// With more blocks than places the early start hides the last wave: as fast at
-// 48^3 FP32 (1.16), 11.8 against 12.1 at 56^3 (1.6), 11.1 against 11.7 at 32^3
-// FP64 (1.6).
+// Whether the plain steps of the whole domain overlap (steps_overlap).
 template <typename S>
-culbm_status inplace_overlap(culbm_sim* s)
+culbm_status plain_overlap(culbm_sim* s)
 {
     using R = typename ArithOf<S>::type;
-    int sms = 0, per_sm = 0;
-    CULBM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev));
-    CULBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_aa_odd<S, R>,
-                                                             AaShape<S>::rows * AaShape<S>::cols, 0));
-    const dim3 g = split_grid(s->dom, AaShape<S>::rows, AaShape<S>::cols);
-    s->inplace_overlap = 4ll * g.x * g.y * g.z > 5ll * sms * per_sm;
+    const Domain& D = s->dom;
+    auto count = [](dim3 g) { return 1ll * g.x * g.y * g.z; };
+    if constexpr (Is16<S>::value) {
+        if (two_cells<S>(D)) {
+            long long blocks = (D.nxy + 2ll * kCells2Threads - 1) / (2ll * kCells2Threads) * D.nz;
+            if (s->inplace) cells2_grid(D, 0, D.nz, &blocks);
+            if (s->inplace)
+                CULBM_CUDA(steps_overlap(s->dev, k_aa_odd_cells2<S, false>, kCells2Threads, blocks, &s->overlap));
+            else
+                CULBM_CUDA(steps_overlap(s->dev, k_pull_cells2<S, false>, kCells2Threads, blocks, &s->overlap));
+            return CULBM_OK;
+        }
+    }
+    if (s->inplace)
+        CULBM_CUDA(steps_overlap(s->dev, k_aa_odd<S, R>, AaShape<S>::rows * AaShape<S>::cols,
+                                 count(split_grid(D, AaShape<S>::rows, AaShape<S>::cols)), &s->overlap));
+    else
+        CULBM_CUDA(steps_overlap(s->dev, k_pull_step<S, R>, 256, count(cell_grid(D)), &s->overlap));
     return CULBM_OK;
 }
 
@@ -1069,8 +1072,7 @@ culbm_status culbm_create(const culbm_config* cfg, culbm_sim** out)
             s->edge_elems = 2 * (fx + fy + fz);
             CULBM_TRY(dev_alloc(s, &s->d_edge, s->edge_elems * s->esize, "edge buffer"));
         }
-        if (inplace)
-            CULBM_TRY(with_storage(s, [&](auto tag) { return inplace_overlap<typename decltype(tag)::type>(s); }));
+        CULBM_TRY(with_storage(s, [&](auto tag) { return plain_overlap<typename decltype(tag)::type>(s); }));
         s->red_blocks = kRedBlocks;
         CULBM_TRY(dev_alloc(s, reinterpret_cast<void**>(&s->d_red), (4ull * s->red_blocks + 4) * sizeof(double),
                             "reduction scratch"));

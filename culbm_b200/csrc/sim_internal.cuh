@@ -64,7 +64,7 @@ struct culbm_sim {
     size_t esize = 4;               // bytes per stored population
     bool inplace = false;           // AA pattern in one buffer; else a double buffer (or the ring)
     bool mixed = false;             // many walls or idle cells (mixed_domain)
-    bool inplace_overlap = true;    // in place: a step's blocks may start while the step before runs
+    bool overlap = true;            // a plain step's blocks may start while the step before runs (steps_overlap)
     double* d_red = nullptr;        // reduction partials
     int red_blocks = 0;
 

@@ -67,7 +67,7 @@ struct StepArgs {
     int ring_nz;   // LAYOUT_PULL_RING: planes in the ring buffer
     int ring_off;  // LAYOUT_PULL_RING: ring plane of domain plane z = 0
     uint32_t seed; // step_seed of the time step being written (stochastic rounding)
-    int overlap;   // in-place: the next step's blocks may start while this one's run (step_enter)
+    int overlap;   // the next step's blocks may start while this one's run (step_enter)
 };
 
 __device__ __forceinline__ int nb_off(const Domain& D, int d)
@@ -240,6 +240,28 @@ __device__ __forceinline__ void step_enter(bool overlap = true)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Whether a step's dependents may start at once: not when nearly the whole
+// grid is resident at once.  The next step's blocks then take their places
+// while this one's run, wherever there is room, and crowd some SMs; a short
+// step waits for its fullest SM.  In us per step, started at once against as
+// blocks end (launched the ordinary way): in place 12^3 FP32 11.7/8.8 (11.3),
+// 96x24x24 12.5/10.2 (12.0), 128x32x32 (1.05 times the resident blocks)
+// 12.1/11.0, 25^3 FP16-SR 11.8/9.9; pull 64x24x24 FP16-SR 5.8/3.3 (5.1),
+// 128x16x16 FP32 5.3/3.1 (5.1), 40^3 FP32 6.1/4.6 (6.2); 40 adjoint forward steps at
+// 64x32x32 FP16-SR 579/366 (509).  With more blocks than places the early start
+// hides the last wave: as fast at 1.1 times the places (64^3 FP16-SR pull 8.5/8.3,
+// 56^3 FP32 pull 7.1/7.1), 11.8/12.1 at 1.6 (56^3 FP32 in place), 63.6/64.7 at
+// 160x120x100 FP16-SR in place.
+template <typename... P>
+cudaError_t steps_overlap(int dev, void (*kernel)(P...), int threads, long long blocks, bool* overlap)
+{
+    int sms = 0, per_sm = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+    *overlap = 4 * blocks > 5ll * sms * per_sm;
+    return e;
+}
+
 // A step launch; `follows`: the launch before it on the stream is a step too.
 template <typename... P, typename... A>
 cudaError_t launch_step(bool follows, dim3 grid, dim3 block, cudaStream_t st, void (*kernel)(P...), const A&... args)
@@ -299,7 +321,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1)
     k_pull_step(const __grid_constant__ StepArgs<S, R> a, int z0)
 {
     const CellCoord c = cell_of_thread(a.dom, z0);
-    step_enter();
+    step_enter(a.overlap != 0);
     if (c.valid) pull_cell<S, R>(a, c);
 }
 

@@ -191,19 +191,21 @@ def test_degenerate_domains_bitwise(culbm, orc, dims):
                 assert_bitwise(sim.pulled_ddf(), want, f"{dims} {policy} {nsteps}")
 
 
+@pytest.mark.parametrize("policy", PLAIN)
 @pytest.mark.parametrize("storage", ["fp32", "fp64", "fp16sr"])
-@pytest.mark.parametrize("dims", [(13, 12, 11), (41, 40, 39), (127, 32, 32), (57, 52, 50), (97, 60, 60)])
-def test_consecutive_inplace_steps_follow_one_another(culbm, storage, dims):
+@pytest.mark.parametrize("dims", [(13, 12, 11), (41, 40, 39), (127, 32, 32), (57, 52, 50), (97, 60, 60), (64, 24, 24),
+                                  (64, 64, 64), (96, 80, 72)])
+def test_consecutive_steps_follow_one_another(culbm, policy, storage, dims):
     """Steps of one call are launched to overlap, those of a grid that is
-    resident at once differently from those of a larger one (96-cell row
-    blocks, 2072 resident for FP32): the bits of steps taken call by call,
-    which do not overlap."""
+    nearly resident at once differently from those of a larger one (of 64^3
+    cells, between 0.7 and 1.4 times the resident blocks): the bits of steps
+    taken call by call, which do not overlap."""
     sc = S.reference_channel_cube(*dims, 0.05)
     got = []
     for calls in ([40], [1] * 40):
-        with make_sim(culbm, dims, (1, 0), storage=storage) as sim:
+        with make_sim(culbm, dims, policy, storage=storage) as sim:
             sim.load_state(*sc.arrays())
             for n in calls:
                 sim.step(n)
             got.append(sim.pulled_ddf(np.float64 if storage == "fp64" else np.float32))
-    assert_bitwise(got[0], got[1], f"{dims} {storage}")
+    assert_bitwise(got[0], got[1], f"{policy} {dims} {storage}")
