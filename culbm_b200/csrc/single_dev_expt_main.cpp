@@ -259,6 +259,12 @@ int run(Options o)
                       << "] gridDim [1,1,1] innerLoop " << t.inner_loop << " (modelled speed-up "
                       << t.predicted_speedup << " over plain streaming, " << t.predicted_speedup_b200
                       << " with B200's measured step costs)" << std::endl;
+            const bool tiled = o.cfg.use_ring_ddf_buf || o.cfg.persist_l2 ||
+                               (o.cfg.opt_policy == CULBM_OPT_L1L2 && o.cfg.stream_policy == CULBM_STREAM_PULL);
+            if (!tiled)
+                std::cout << "  (without --useRingDDFBuf or --persistL2 this policy runs as plain pull steps: the tile "
+                             "takes no part)"
+                          << std::endl;
         }
     }
     if (o.dstep == 0) throw std::invalid_argument("--dstep must be positive");

@@ -64,3 +64,17 @@ def test_addition_flags_parse(flag):
     assert r.returncode == 1, (r.returncode, r.stderr)
     assert "Dimension of domain doesn't match computation grid!" in r.stderr
     assert "--persistL2" in run("--help").stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("args,tiled", [(["--streamPolicy", "1", "--optPolicy", "3"], False),
+                                        (["--streamPolicy", "1", "--optPolicy", "3", "--useRingDDFBuf"], True),
+                                        (["--streamPolicy", "0", "--optPolicy", "1", "--persistL2"], True),
+                                        (["--streamPolicy", "0", "--optPolicy", "2"], True),
+                                        (["--streamPolicy", "1", "--optPolicy", "2"], False)])
+def test_auto_tile_says_whether_it_is_used(args, tiled, tmp_path):
+    r = run("--blockDim", "auto", "--domainDim", "[128,96,96]", "--nstep", "2", "--dstep", "2", "--dumpFolder",
+            str(tmp_path), *args)
+    assert r.returncode == 0, r.stderr
+    assert "Auto tile: blockDim" in r.stdout
+    assert ("takes no part" in r.stdout) == (not tiled)
