@@ -243,12 +243,22 @@ def fp64_errors(culbm, steps=1000):
                         f"{steps} steps, vs FP64 storage+arithmetic", "errors": out}
 
 
+def executed(op, launches):
+    """What a blocked leg ran, for its `policy` text: without the ring buffer or
+    the persisting-L2 window, optPolicy 1 and 3 step as plain pulls, one launch
+    each, and the tile takes no part."""
+    if not op:
+        return ""
+    return ", run as plain pull steps" if launches == 1.0 else ", run on the L2 tile engine"
+
+
 def selector_summary(sel):
     """culbm_select_tile's pick: the model's speed-up over plain streaming
     (the reference's model, with the 16-bit compute floor), the same tile's
     speed-up with B200's measured step costs, and whether blocking is
     expected to pay (the latter above 1).  --blockDim auto with a blocked
-    optPolicy prints both."""
+    optPolicy prints both, of a tile that only the ring buffer, the
+    persisting-L2 window and optPolicy 2 with pull streaming use."""
     return {"tile": list(sel["tile"]), "inner_loop": sel["inner_loop"],
             "predicted_speedup": round(sel["speedup"], 4),
             "predicted_speedup_b200": round(sel["speedup_b200"], 4),
@@ -257,7 +267,7 @@ def selector_summary(sel):
 
 def mixed_precision_512(culbm, steps):
     """The 512x512x256 channel with 120 spheres (radii 6-18): in-place
-    streaming with FP32, FP16 and BF16 storage, plain and L2-blocked."""
+    streaming with FP32, FP16 and BF16 storage, and optPolicy 3."""
     from culbm_b200 import scenes
     sc = scenes.spheres_512()
     peak, _ = peaks()
@@ -276,11 +286,12 @@ def mixed_precision_512(culbm, steps):
         "blocked_inplace_fp16sr": (3, "fp16sr", tuple(s16["tile"]), s16["inner_loop"]),
     }.items():
         try:
-            mlups, mps, _ = measure(culbm, sc, 1, op, st, steps, 3, tile=tile, inner=inner)
+            mlups, mps, inf = measure(culbm, sc, 1, op, st, steps, 3, tile=tile, inner=inner)
             out["runs"][name] = {"mlups": round(mlups, 1), "ms_per_step": round(mps, 4),
                                  "hbm_frac_of_measured": round(mlups * 1e6 * BYTES_PER_LUP[st] / 1e9 / peak, 4),
                                  "policy": "streamPolicy 1, optPolicy %d" % op +
-                                           (f", tile {tile} (culbm_select_tile), innerLoop {inner}" if op else "")}
+                                           (f", tile {tile} (culbm_select_tile), innerLoop {inner}" if op else "") +
+                                           executed(op, inf.get("launches_per_step"))}
         except Exception as e:   # report, do not hide
             out["runs"][name] = {"error": str(e)}
     return out
@@ -556,10 +567,11 @@ def run_ours(args):
         "inplace_bf16": (1, 0, "bf16", None, 5),
         "pull_fp16": (0, 0, "fp16", None, 5),
         "pull_fp16sr": (0, 0, "fp16sr", None, 5),
-        # the reference README's (1,3) launch shape: tile [32,16,2] x [2,6,38]
+        # the reference README's (1,3) launch shape, tile [32,16,2] x [2,6,38], and the selector's;
+        # both run as plain pull steps, which `policy` says
         "blocked_inplace_fp32_readme_tile": (1, 3, "fp32", (64, 96, 76), 5),
         "blocked_inplace_fp32_selected_tile": (1, 3, "fp32", tuple(sel["tile"]), sel["inner_loop"]),
-        # (0,3): pull L2 tiles, the same two tiles
+        # (0,3): the same two tiles, plain pull steps again
         "blocked_pull_fp32_readme_tile": (0, 3, "fp32", (64, 96, 76), 5),
         "blocked_pull_fp32_selected_tile": (0, 3, "fp32", tuple(sel["tile"]), sel["inner_loop"]),
         # (0,2): the cluster engine, tile 32x8x16 as 16 CTAs of 32x4x2 cells
@@ -575,7 +587,8 @@ def run_ours(args):
                            "hbm_frac_of_measured": round(mlups * 1e6 * BYTES_PER_LUP[st] / 1e9 / peak, 4),
                            "policy": f"streamPolicy {sp}, optPolicy {op}" +
                                      (f", tile {tile}, innerLoop {inner}" if op else "") +
-                                     (f", CTA {split[0]} x cluster {split[1]}" if split else ""),
+                                     (f", CTA {split[0]} x cluster {split[1]}, run on the cluster engine" if split
+                                      else executed(op, inf.get("launches_per_step"))),
                            "launches_per_step": inf.get("launches_per_step"),
                            "clocks": inf.get("clocks")}
         except Exception as e:   # report, do not hide
