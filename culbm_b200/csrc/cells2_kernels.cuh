@@ -5,7 +5,7 @@
 // instructions per cell of the FP16-SR pull, against half the bytes of FP32.
 // Two cells in one row share every address and, with even nx, an aligned
 // 32-bit word of every plane, and their collision runs in packed FP32
-// (packed2.cuh): 453 instructions per cell.  The pulled values stay in their
+// (packed2.cuh): 457 instructions per cell.  The pulled values stay in their
 // stored form and are widened twice, once for the moments and once for the
 // relaxation, and each pair of directions is narrowed and stored as soon as
 // it is relaxed, so that the two cells run at 80 registers (six blocks of 128;

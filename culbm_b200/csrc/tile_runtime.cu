@@ -111,7 +111,7 @@ bool is_blocked(const culbm_config& cfg) { return cfg.opt_policy != CULBM_OPT_NO
 // the plain pull does, so the choice is one of speed.  B200's L2 copies only
 // twice as fast as its HBM: at 288x272x280 the tile engine reached 15.0k
 // MLUPS with the README tile (FP32) and at most 24.3k with any, the plain
-// pull 29.7k; FP16-SR tiles 19.2k against 38.7k.  The tile engine stays where
+// pull 29.7k; FP16-SR tiles 19.2k against 46.1k.  The tile engine stays where
 // the caller asks for something only it does: the ring buffer (one population
 // buffer), the persisting-L2 window, and optPolicy 2 with pull streaming (its
 // cluster engine, or L2 tiles where no cluster holds the tile).

@@ -52,7 +52,7 @@ typedef enum culbm_stream_policy { CULBM_STREAM_PULL = 0, CULBM_STREAM_INPLACE =
  * 16 CTAs), and tiles no cluster holds on the L2 tile engine.  The other
  * blocked policies run on the L2 tile engine with use_ring_ddf_buf or
  * persist_l2, and else as plain pull steps between two population buffers,
- * which B200 takes 1.2 to 2 times as fast. */
+ * which B200 takes 1.2 to 2.4 times as fast. */
 typedef enum culbm_opt_policy {
     CULBM_OPT_NONE = 0,
     CULBM_OPT_STATIC_L2 = 1,
@@ -301,7 +301,9 @@ typedef struct culbm_tile_choice {
     double predicted_speedup_no_alignment;  /* the same without the sector-alignment term (S0) */
     double predicted_speedup_b200; /* S of the chosen tile with B200's measured step costs
                                       (CULBM_B200_PLAIN_* and CULBM_B200_TILE_*): above 1 when
-                                      blocking is expected to beat plain streaming on B200 */
+                                      blocking is expected to beat plain streaming on B200.  Of the
+                                      tile engine: optPolicy 1 and 3, and 2 in place, run on it with
+                                      use_ring_ddf_buf or persist_l2 only */
     uint32_t reserved[6];
 } culbm_tile_choice;
 
@@ -309,13 +311,14 @@ typedef struct culbm_tile_choice {
  * (DRAM copy 6.48 TB/s, L2 copy 13.4 TB/s; a partial sector costs 8.8 full ones). */
 #define CULBM_B200_LAMBDA 0.4841
 #define CULBM_B200_GAMMA 8.772
-/* The 16-bit formats' plain step is bound by instruction issue, not DRAM: its
- * time per update over the DRAM time of its 108 bytes at the copy bandwidth
- * (FP16-SR pull: 36.2k MLUPS against 60.6k) on a B200.  The model takes the
+/* The 16-bit formats' plain step is bound by instruction issue and latency, not
+ * DRAM: its time per update over the DRAM time of its 108 bytes at the copy
+ * bandwidth (FP16-SR pull, even nx: 46.1k MLUPS against 60.6k; odd nx keeps one
+ * cell per thread, 35.4k and 1.71) on a B200.  The model takes the
  * larger of memory and compute time per update, so for these formats every
  * blocked tile predicts S < 1 (the halo cells cost compute and save only
  * bandwidth) and the tile of largest S is the one with the least halo. */
-#define CULBM_B200_COMPUTE_16 1.67
+#define CULBM_B200_COMPUTE_16 1.32
 /* Measured step costs on B200, each as time per update over the DRAM time of
  * the format's bytes per update at the copy bandwidth.  The model takes the
  * DRAM traffic of an L2-blocked round as its time; on B200 the tile steps
