@@ -419,29 +419,39 @@ bool two_cells(const Domain& D)
 // pull, 303/307, 311/307, 318/306 and 334/305 in place (FP16: 247/237 and
 // 293/287 at 10 %); idle planes 20 % 212/207 and 249/257, 30 % 201/187 and
 // 229/231; planes of walls 30 % 245/242 and 286/302.
-// 512 segments of the caller's flags, spread over the domain, are looked at (all
-// where there are no more): 10 us of a load, and an estimate is enough for a speed.
+// 128 segments of the caller's flags, spread over the domain, are looked at (all
+// where there are no more), while the inputs are on their way to the device: an
+// estimate is enough for a speed.
 bool mixed_domain(const culbm_sim* s, const uint32_t* flag)
 {
     const Domain& D = s->dom;
     if (flag == nullptr || s->esize != 2 || D.nx % 2 != 0) return false;   // NULL: fluid everywhere
-    const uint64_t row = (static_cast<uint64_t>(D.nx) + 31) / 32, all = row * D.ny * D.nz;
-    const uint64_t looks = std::min<uint64_t>(all, 512);
-    uint64_t found = 0;
-    for (uint64_t k = 0; k < looks; ++k) {
+    const uint32_t row = (static_cast<uint32_t>(D.nx) + 31) / 32, all = row * static_cast<uint32_t>(D.ny) * D.nz;
+    const uint32_t looks = std::min<uint32_t>(all, 128);
+    uint32_t found = 0;
+    for (uint32_t k = 0; k < looks; ++k) {
         // fractional parts of multiples of the golden ratio: even, and in step with no row or plane
-        const uint64_t seg = all == looks ? k : (k * 0x9E3779B97F4A7C15ull >> 32) * all >> 32;
-        const int x0 = static_cast<int>(seg % row) * 32;
-        const uint32_t* f = flag + seg / row * D.nx + x0;
-        bool flow = false, wall = false, other = false, idle = true;
-        for (int x = 0; x < std::min(32, D.nx - x0); ++x) {
-            const bool moves = (f[x] & (FLAG_COLLIDE | FLAG_EQU)) != 0;
-            flow = flow || moves;
-            other = other || !moves;
-            wall = wall || (!moves && (f[x] & FLAG_STORE));
-            idle = idle && !(f[x] & (FLAG_LOAD | FLAG_EQU));
-        }
-        found += s->inplace ? (wall && flow) || idle : other;
+        const uint32_t seg =
+            all == looks ? k : static_cast<uint32_t>(static_cast<uint64_t>(k * 0x9E3779B9u) * all >> 32);
+        const uint32_t line = seg / row, x0 = (seg - line * row) * 32;
+        const uint32_t* f = flag + static_cast<size_t>(line) * D.nx + x0;
+        // in bit 0: a cell that collides or takes an equilibrium, one that does neither, one of those that
+        // stores, one that loads or takes an equilibrium
+        uint32_t flow = 0, other = 0, wall = 0, busy = 0;
+        auto look = [&](uint32_t v) {
+            const uint32_t moves = v >> 2 | v >> 1;
+            flow |= moves;
+            other |= ~moves;
+            wall |= ~moves & v >> 4;
+            busy |= v | v >> 1;
+        };
+        static_assert(FLAG_LOAD == 1u && FLAG_EQU == 2u && FLAG_COLLIDE == 4u && FLAG_STORE == 16u);
+        const int n = std::min(32, D.nx - static_cast<int>(x0));
+        if (n == 32)
+            for (int x = 0; x < 32; ++x) look(f[x]);
+        else
+            for (int x = 0; x < n; ++x) look(f[x]);
+        found += s->inplace ? ((wall & flow) | ~busy) & 1u : other & 1u;
     }
     return (s->inplace ? 5 : 6) * found > looks;
 }
@@ -690,7 +700,6 @@ culbm_status upload_state(culbm_sim* s, const uint32_t* flag, const float* const
 {
     const long long n = s->n;
     const dim3 g1(1184), b1(256);
-    s->mixed = mixed_domain(s, flag);
     if (flag != nullptr) {
         CULBM_CUDA(cudaMemcpyAsync(s->d_flag, flag, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
     } else {
@@ -709,6 +718,7 @@ culbm_status upload_state(culbm_sim* s, const uint32_t* flag, const float* const
     k_build_ops<<<cell_grid(s->dom), cell_block(), 0, s->stream>>>(s->dom, s->d_flag, s->d_ops, 0);
     CULBM_CUDA(cudaGetLastError());
     CULBM_TRY(with_storage(s, [&](auto tag) { return fill_rest<typename decltype(tag)::type>(s); }));
+    s->mixed = mixed_domain(s, flag);
     s->step = 0;
     s->loaded = true;
     return CULBM_OK;
@@ -900,7 +910,6 @@ culbm_status run_host_overlapped(culbm_sim* s, const uint32_t* flag, const float
     cudaStream_t h2d = s->copy_st[0], d2h = s->copy_st[1];
     const int T = static_cast<int>(nsteps);
 
-    s->mixed = mixed_domain(s, flag);
     // Everything follows the simulation's earlier work.
     CULBM_CUDA(cudaEventRecord(s->run_ev[0], s->stream));
     CULBM_CUDA(cudaStreamWaitEvent(h2d, s->run_ev[0], 0));
@@ -932,6 +941,8 @@ culbm_status run_host_overlapped(culbm_sim* s, const uint32_t* flag, const float
                                            h2d));
         CULBM_CUDA(cudaEventRecord(ev(j, kSlabIn), h2d));
     }
+
+    s->mixed = mixed_domain(s, flag);
 
     // Slab by slab for the first and the last nslab steps, which the copies
     // overlap; whole-domain launches in between.  fill_rest left cur = 0 and
